@@ -30,8 +30,9 @@ struct LaunchSizes
 {
         long long extend_blocks = 1;
         long long shadow_blocks = 1;
-        long long extend_refill_blocks[3] = {1, 1, 1};  // per staging chunk: 1, 2, 4 rounds of 32 tests
-        long long shadow_refill_blocks[3] = {1, 1, 1};
+        // per walk variant: direct loads, then staging chunks of 1, 2, 4 rounds of 32 tests
+        long long extend_refill_blocks[4] = {1, 1, 1, 1};
+        long long shadow_refill_blocks[4] = {1, 1, 1, 1};
         long long stream_blocks = 1;
 };
 
