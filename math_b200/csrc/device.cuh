@@ -4,6 +4,7 @@
 #pragma once
 
 #include "device_types.h"
+#include "walk_math.hpp"
 
 #include <cfloat>
 #include <cstdint>
@@ -366,90 +367,96 @@ __device__ __noinline__ Leaf<N> find_leaf_dfs(const MeshDev<N>& M, const Point<N
 #endif
 constexpr int WALK_BLOCK = NT_BLOCK;
 
-// The root-to-leaf path of the previous point location of the same walk.  Consecutive leaves of a
-// walk share most of their ancestors; the child chosen at each level depends only on the point and
-// the box origins above it, so while the new point picks the same children the node records are
-// known and are not read again.  The leaf found is the one a full descent finds.
+// The root-to-leaf path of the previous point location of the same lane: the finest-level cell of the
+// located point (its indices along the axes, TreeBits<N>::D bits each) and the leaf that holds it.  A
+// new point shares the path down to the first level at which an index bit differs, so its descent
+// starts there: the first child of the internal node at each level of the path is kept in shared memory
+// (path_cache_slots).
 struct PathCache
 {
-        int depth;                 // level of the cached leaf; -1: empty
-        int2 leaf;                 // the cached leaf's record
-        // the first child of the internal node at each level of the path, and the child chosen there,
-        // are kept in shared memory (path_cache_slots, path_cache_child)
+        int depth;      // level of the cached leaf; -1: empty
+        int2 leaf;      // the cached leaf's record
+        unsigned code;  // the cell indices, axis i at bit i x D
 
         __device__ __forceinline__ void reset()
         {
                 depth = -1;
+                leaf = make_int2(0, 0);
+                code = 0;
         }
 };
 
-// This thread's column of the block's path-cache slots (MAX_LEVELS x WALK_BLOCK ints).
+// This thread's column of the block's path-cache slots (one per internal level x WALK_BLOCK ints).
+template <int N>
 __device__ __forceinline__ int* path_cache_slots()
 {
-        __shared__ int s_fc[MAX_LEVELS * WALK_BLOCK];
+        __shared__ int s_fc[TreeBits<N>::D * WALK_BLOCK];
         return s_fc + threadIdx.x;
 }
 
-// This thread's column of the child indices chosen along the cached path (MAX_LEVELS x WALK_BLOCK
-// bytes; consecutive threads share 32-bit words, which costs no bank conflicts).
-__device__ __forceinline__ unsigned char* path_cache_child()
+// The block's copy of the mesh's boundary table (every thread of the block calls it once, before the
+// first walk).
+template <int N>
+__device__ __forceinline__ const float* walk_bounds(const MeshDev<N>& M)
 {
-        __shared__ unsigned char s_child[MAX_LEVELS * WALK_BLOCK];
-        return s_child + threadIdx.x;
+        constexpr int COUNT = N * (TreeBits<N>::CELLS + 1);
+        __shared__ float s_bounds[COUNT];
+        for (int i = threadIdx.x; i < COUNT; i += blockDim.x)
+        {
+                s_bounds[i] = __ldg(M.bounds + i);
+        }
+        __syncthreads();
+        return s_bounds;
 }
 
 template <int N>
-__device__ __forceinline__ bool find_leaf_cached(const MeshDev<N>& M, const float* p, PathCache& pc, Leaf<N>* out,
-                                                 int2* leaf_rec, unsigned* descent)
+struct Located
 {
-        int* const fc = path_cache_slots();
-        unsigned char* const cc = path_cache_child();
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-        {
-                if (!(p[i] <= M.root_d1[i]) || !(-p[i] <= -M.root_org[i]))
-                {
-                        return false;
-                }
-        }
+        Leaf<N> leaf;
+        int2 rec;
+        int levels;  // nodes visited
+};
+
+// The exact descent from the root, for points that lie on a box boundary or within near_bound of one.
+// Out of line and by value, as find_leaf_dfs.
+template <int N>
+__device__ __noinline__ Located<N> locate_exact(const MeshDev<N>& M, const Point<N> pt)
+{
+        Located<N> res;
+        res.leaf.node = -1;
+        res.leaf.level = 0;
+        res.rec = make_int2(0, 0);
+        res.levels = 0;
         float o[N];
+        bool outside = false;
 #pragma unroll
         for (int i = 0; i < N; ++i)
         {
                 o[i] = M.root_org[i];
+                res.leaf.org[i] = 0;
+                outside |= !(pt.v[i] <= M.root_d1[i]) || !(-pt.v[i] <= -M.root_org[i]);
+        }
+        if (outside)
+        {
+                return res;
         }
         int node = 0;
         bool ambiguous = false;
-        bool same = pc.depth >= 0;
         for (int lvl = 0; lvl < MAX_LEVELS; ++lvl)
         {
-                int2 nd;
-                if (same)
-                {
-                        nd = (lvl == pc.depth) ? pc.leaf : make_int2(fc[lvl * WALK_BLOCK], -1);
-                }
-                else
-                {
-                        nd = __ldg(&M.nodes[node]);
-                }
-                ++*descent;
+                const int2 nd = __ldg(&M.nodes[node]);
+                ++res.levels;
                 if (nd.y >= 0)
                 {
-                        out->node = node;
-                        out->level = lvl;
+                        res.leaf.node = node;
+                        res.leaf.level = lvl;
 #pragma unroll
                         for (int i = 0; i < N; ++i)
                         {
-                                out->org[i] = o[i];
+                                res.leaf.org[i] = o[i];
                         }
-                        *leaf_rec = nd;
-                        pc.depth = lvl;
-                        pc.leaf = nd;
-                        return true;
-                }
-                if (!same)
-                {
-                        fc[lvl * WALK_BLOCK] = nd.x;
+                        res.rec = nd;
+                        return res;
                 }
                 int child = 0;
                 bool fail = false;
@@ -458,8 +465,8 @@ __device__ __forceinline__ bool find_leaf_cached(const MeshDev<N>& M, const floa
                 {
                         float h = M.size[lvl + 1][i];
                         float mid = o[i] + h;
-                        bool lo_ok = p[i] <= mid;
-                        bool hi_ok = (-p[i] <= -mid) && (p[i] <= mid + h);
+                        bool lo_ok = pt.v[i] <= mid;
+                        bool hi_ok = (-pt.v[i] <= -mid) && (pt.v[i] <= mid + h);
                         if (lo_ok)
                         {
                                 ambiguous |= hi_ok;
@@ -476,33 +483,185 @@ __device__ __forceinline__ bool find_leaf_cached(const MeshDev<N>& M, const floa
                 }
                 if (fail)
                 {
-                        pc.depth = -1;
                         if (ambiguous)
                         {
-                                Point<N> pt;
-#pragma unroll
-                                for (int i = 0; i < N; ++i)
+                                res.leaf = find_leaf_dfs<N>(M, pt);
+                                if (res.leaf.node >= 0)
                                 {
-                                        pt.v[i] = p[i];
-                                }
-                                *out = find_leaf_dfs<N>(M, pt);
-                                if (out->node >= 0)
-                                {
-                                        *leaf_rec = __ldg(&M.nodes[out->node]);
-                                        return true;
+                                        res.rec = __ldg(&M.nodes[res.leaf.node]);
                                 }
                         }
-                        return false;
-                }
-                if (!same || (int)cc[lvl * WALK_BLOCK] != child)
-                {
-                        same = false;
-                        cc[lvl * WALK_BLOCK] = (unsigned char)child;
+                        return res;
                 }
                 node = nd.x + child;
         }
-        pc.depth = -1;
-        return false;
+        return res;
+}
+
+// The leaf that contains p (find_box_for_point, tree.h:441-463): the path to it is the bits of its finest
+// cell (point_cell, `bounds` the mesh's table in shared or global memory), and nodes are read only from
+// the first level at which that path leaves the cached one.  Points at a box boundary take the exact
+// descent.  *descent counts the levels of the full descent, which is the algorithm's work.
+template <int N>
+__device__ __forceinline__ bool locate_leaf(const MeshDev<N>& M, const float* bounds, const float* p, PathCache& pc,
+                                            Leaf<N>* out, int2* leaf_rec, unsigned* descent)
+{
+        constexpr int D = TreeBits<N>::D;
+        constexpr int CELLS = TreeBits<N>::CELLS;
+        unsigned code;
+        const CellResult cell = point_cell<N>(bounds, M.root_org, M.inv_cell, M.near_bound, p, &code);
+        if (cell == CELL_NEAR)
+        {
+                Point<N> pt;
+#pragma unroll
+                for (int i = 0; i < N; ++i)
+                {
+                        pt.v[i] = p[i];
+                }
+                const Located<N> r = locate_exact<N>(M, pt);
+                *descent += r.levels;
+                *out = r.leaf;
+                *leaf_rec = r.rec;
+                return r.leaf.node >= 0;
+        }
+        if (cell == CELL_OUTSIDE)
+        {
+                return false;
+        }
+        int* const fc = path_cache_slots<N>();
+        // levels whose index bits agree in every axis
+        int lvl = D - (32 - __clz(cell_difference<N>(code, pc.code)));
+        int2 nd = pc.leaf;
+        if (lvl >= pc.depth)
+        {
+                if (pc.depth < 0)
+                {
+                        nd = __ldg(&M.nodes[0]);
+                        lvl = 0;
+                        if (nd.y < 0)
+                        {
+                                fc[0] = nd.x;
+                        }
+                }
+                else
+                {
+                        lvl = pc.depth;
+                }
+        }
+        else
+        {
+                nd = make_int2(fc[lvl * WALK_BLOCK], -1);
+        }
+        while (nd.y < 0)
+        {
+                nd = __ldg(&M.nodes[nd.x + (int)child_bits<N>(code, D - 1 - lvl)]);
+                ++lvl;
+                if (nd.y < 0)
+                {
+                        if (lvl >= D)
+                        {
+                                // deeper than the depth limit: not a tree this library builds
+                                pc.depth = -1;
+                                return false;
+                        }
+                        fc[lvl * WALK_BLOCK] = nd.x;
+                }
+        }
+        pc.code = code;
+        pc.depth = lvl;
+        pc.leaf = nd;
+        *leaf_rec = nd;
+        *descent += lvl + 1;
+        out->node = 0;
+        out->level = lvl;
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+        {
+                const unsigned c = (code >> (i * D)) & (CELLS - 1);
+                out->org[i] = bounds[i * (CELLS + 1) + ((c >> (D - lvl)) << (D - lvl))];
+        }
+        return true;
+}
+
+// ------------------------------------------------------------------------------------------------
+// The exit from a leaf (leaf_exit_fast; the exact routine where that cannot decide)
+
+template <int N>
+struct BoxStep
+{
+        float org[N], size[N], cur[N], dir[N];
+};
+
+template <int N>
+__device__ __noinline__ Exit<N> leaf_exit_exact(const BoxStep<N> b)
+{
+        Exit<N> x;
+        float first_t, second_t;
+        x.ok = box_slabs<N>(b.org, b.size, b.cur, b.dir, &first_t, &second_t);
+        x.t = second_t;
+        x.nudge = 0;
+        float d1[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+        {
+                x.ip[i] = b.cur[i] + b.dir[i] * second_t;
+                d1[i] = b.org[i] + b.size[i];
+        }
+        if (x.ok)
+        {
+                int ax;
+                float sg;
+                box_normal_axis<N>(b.org, d1, x.ip, &ax, &sg);
+                x.nudge = sg > 0 ? ax + 1 : -(ax + 1);
+        }
+        return x;
+}
+
+struct DeviceQuotient
+{
+        static __device__ __forceinline__ float rcp(float x)
+        {
+                float r;
+                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+                return r;
+        }
+        static __device__ __forceinline__ float div(float a, float b)
+        {
+                return __fdiv_rn(a, b);
+        }
+};
+
+template <int N>
+__device__ __forceinline__ Exit<N> leaf_exit(const float* org, const float* size, const float* cur, const float* dir)
+{
+        Exit<N> x;
+        if (!leaf_exit_fast<N, DeviceQuotient>(org, size, cur, dir, &x))
+        {
+                BoxStep<N> b;
+#pragma unroll
+                for (int i = 0; i < N; ++i)
+                {
+                        b.org[i] = org[i];
+                        b.size[i] = size[i];
+                        b.cur[i] = cur[i];
+                        b.dir[i] = dir[i];
+                }
+                x = leaf_exit_exact<N>(b);
+        }
+        return x;
+}
+
+// The size of the boxes at a level: the root's halved per level (exact), without an indexed read of the
+// parameters that differs from lane to lane.
+template <int N>
+__device__ __forceinline__ void level_size(const MeshDev<N>& M, int level, float* size)
+{
+        const float scale = __int_as_float((127 - level) << 23);
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+        {
+                size[i] = M.size[0][i] * scale;
+        }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -883,10 +1042,11 @@ __device__ bool mesh_closest(const MeshDev<N>& M, const Ray<N>& ray, float root_
         {
                 Leaf<N> lf;
                 int2 nd;
-                if (find_leaf_cached<N>(M, probe, pc, &lf, &nd, &ws->descent))
+                if (locate_leaf<N>(M, M.bounds, probe, pc, &lf, &nd, &ws->descent))
                 {
                         ++ws->box_steps;
-                        const float* sz = M.size[lf.level];
+                        float sz[N];
+                        level_size<N>(M, lf.level, sz);
                         if (travelled > tmax * 1.00001f + 1e-6f)
                         {
                                 return false;
@@ -917,28 +1077,20 @@ __device__ bool mesh_closest(const MeshDev<N>& M, const Ray<N>& ray, float root_
                                         }
                                 }
                         }
-                        float first_t, second_t;
-                        if (!box_slabs<N>(lf.org, sz, cur, ray.dir, &first_t, &second_t))
+                        const Exit<N> ex = leaf_exit<N>(lf.org, sz, cur, ray.dir);
+                        if (!ex.ok)
                         {
                                 return false;
                         }
-                        float ip[N], d1[N];
+                        const int ax = (ex.nudge > 0 ? ex.nudge : -ex.nudge) - 1;
+                        const float nudge = ex.nudge > 0 ? M.dist : -M.dist;
 #pragma unroll
                         for (int i = 0; i < N; ++i)
                         {
-                                ip[i] = cur[i] + ray.dir[i] * second_t;
-                                d1[i] = lf.org[i] + sz[i];
+                                cur[i] = ex.ip[i];
+                                probe[i] = (i == ax) ? ex.ip[i] + nudge : ex.ip[i];
                         }
-                        int ax;
-                        float sg;
-                        box_normal_axis<N>(lf.org, d1, ip, &ax, &sg);
-#pragma unroll
-                        for (int i = 0; i < N; ++i)
-                        {
-                                cur[i] = ip[i];
-                                probe[i] = (i == ax) ? ip[i] + M.dist * sg : ip[i] + M.dist * 0.0f;
-                        }
-                        travelled += second_t;
+                        travelled += ex.t;
                 }
                 else
                 {
@@ -1255,8 +1407,30 @@ enum WalkStatus : int
         W_MISS = 2
 };
 
+// Enters the tree from outside, through the root box at the entry distance `travelled` holds.
 template <int N>
-__device__ __forceinline__ void walk_begin(Walk<N>& w, const Ray<N>& ray, float root_t, float tmax)
+__device__ __forceinline__ void walk_enter(const MeshDev<N>& M, Walk<N>& w)
+{
+        float ip[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+        {
+                ip[i] = w.cur[i] + w.ray.dir[i] * w.travelled;
+        }
+        int ax;
+        float sg;
+        box_normal_axis<N>(M.root_org, M.root_d1, ip, &ax, &sg);
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+        {
+                w.cur[i] = ip[i];
+        }
+        // next probe: ip - dist * sg along the entry face's axis
+        w.nudge = sg > 0 ? -(ax + 1) : ax + 1;
+}
+
+template <int N>
+__device__ __forceinline__ void walk_begin(const MeshDev<N>& M, Walk<N>& w, const Ray<N>& ray, float root_t, float tmax)
 {
         w.ray = ray;
         w.ao = 0;
@@ -1271,6 +1445,18 @@ __device__ __forceinline__ void walk_begin(Walk<N>& w, const Ray<N>& ray, float 
         w.steps = 0;
         w.nudge = 0;
         w.raw = 0;
+        bool inside = true;
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+        {
+                inside = inside && ray.org[i] <= M.root_d1[i] && -ray.org[i] <= -M.root_org[i];
+        }
+        if (!inside)
+        {
+                // no leaf holds the origin: the walk's first step, taken here
+                walk_enter<N>(M, w);
+                w.steps = 1;
+        }
         // the path cache describes a root-to-leaf path of the tree, not the ray: it stays valid
         // from one ray of the lane to the next (neighbouring rays share their upper levels), so it
         // is reset once per lane (w.pc.reset()) and not here
@@ -1572,7 +1758,7 @@ __device__ __forceinline__ int leaf_closest_warp(const MeshDev<N>& M, int start,
 // walk_step with the leaf's facets tested by leaf_closest_warp.  Every lane of the warp calls it
 // (active = false for lanes without a walk, whose result is ignored).
 template <int N, int RR = StageFit<N>::ROUNDS>
-__device__ __forceinline__ int walk_step_warp(const MeshDev<N>& M, Walk<N>& w, bool active, int retest,
+__device__ __forceinline__ int walk_step_warp(const MeshDev<N>& M, const float* bounds, Walk<N>& w, bool active, int retest,
                                               const float* raw_org, const float* raw_dir, float* t_out, int* facet_out,
                                               WalkStats* ws, int small_leaf = SMALL_LEAF)
 {
@@ -1590,7 +1776,7 @@ __device__ __forceinline__ int walk_step_warp(const MeshDev<N>& M, Walk<N>& w, b
                         ws->error |= ERR_WALK_LIMIT;
                         status = W_MISS;
                 }
-                else if (find_leaf_cached<N>(M, probe, w.pc, &lf, &nd, &ws->descent))
+                else if (locate_leaf<N>(M, bounds, probe, w.pc, &lf, &nd, &ws->descent))
                 {
                         ++ws->box_steps;
                         if (w.steps == 1)
@@ -1618,7 +1804,8 @@ __device__ __forceinline__ int walk_step_warp(const MeshDev<N>& M, Walk<N>& w, b
         }
         if (leaf)
         {
-                const float* sz = M.size[lf.level];
+                float sz[N];
+                level_size<N>(M, lf.level, sz);
                 if (f >= 0)
                 {
                         float pt[N];
@@ -1640,29 +1827,19 @@ __device__ __forceinline__ int walk_step_warp(const MeshDev<N>& M, Walk<N>& w, b
                                 return W_HIT;
                         }
                 }
-                float first_t, second_t;
-                if (!box_slabs<N>(lf.org, sz, w.cur, w.ray.dir, &first_t, &second_t))
+                const Exit<N> ex = leaf_exit<N>(lf.org, sz, w.cur, w.ray.dir);
+                if (!ex.ok)
                 {
                         return W_MISS;
                 }
-                float ip[N], d1[N];
 #pragma unroll
                 for (int i = 0; i < N; ++i)
                 {
-                        ip[i] = w.cur[i] + w.ray.dir[i] * second_t;
-                        d1[i] = lf.org[i] + sz[i];
-                }
-                int ax;
-                float sg;
-                box_normal_axis<N>(lf.org, d1, ip, &ax, &sg);
-#pragma unroll
-                for (int i = 0; i < N; ++i)
-                {
-                        w.cur[i] = ip[i];
+                        w.cur[i] = ex.ip[i];
                 }
                 // next probe: ip + dist * sg along the exit face's axis
-                w.nudge = sg > 0 ? ax + 1 : -(ax + 1);
-                w.travelled += second_t;
+                w.nudge = ex.nudge;
+                w.travelled += ex.t;
         }
         else
         {
@@ -1670,24 +1847,9 @@ __device__ __forceinline__ int walk_step_warp(const MeshDev<N>& M, Walk<N>& w, b
                 {
                         return W_MISS;
                 }
-                // outside the tree at the start: enter through the root box (travelled holds the
-                // entry distance)
-                float ip[N];
-#pragma unroll
-                for (int i = 0; i < N; ++i)
-                {
-                        ip[i] = w.cur[i] + w.ray.dir[i] * w.travelled;
-                }
-                int ax;
-                float sg;
-                box_normal_axis<N>(M.root_org, M.root_d1, ip, &ax, &sg);
-#pragma unroll
-                for (int i = 0; i < N; ++i)
-                {
-                        w.cur[i] = ip[i];
-                }
-                // next probe: ip - dist * sg along the entry face's axis
-                w.nudge = sg > 0 ? -(ax + 1) : ax + 1;
+                // the origin is inside the root box but in no leaf (a gap between boxes): enter as from
+                // outside
+                walk_enter<N>(M, w);
         }
         return W_RUNNING;
 }

@@ -49,6 +49,15 @@ struct Rec64
         static constexpr int OFF_PLANES = 2 * N;
 };
 
+// The mesh trees' depth limit (boxes per axis 2^TreeBits<N>::D at the finest level; mesh.cpp's maximum
+// depths 10, 8, 6, 5 count the root).
+template <int N>
+struct TreeBits
+{
+        static constexpr int D = N == 3 ? 9 : (N == 4 ? 7 : (N == 5 ? 5 : 4));
+        static constexpr int CELLS = 1 << D;
+};
+
 template <int N>
 struct MeshDev
 {
@@ -71,6 +80,12 @@ struct MeshDev
         float root_d1[N];
         float size[MAX_LEVELS][N];  // box size at depth k (root k = 0)
         float dist;                 // distance_from_facet of the tree (tree.h:419)
+        // point location by arithmetic (locate_leaf): per axis the CELLS + 1 finest box boundaries (the
+        // origins a descent computes, the root box's far plane last), cells per unit length, and the
+        // distance from a boundary within which a point is located by the exact descent instead
+        const float* bounds;        // N x (CELLS + 1)
+        float inv_cell[N];
+        float near_bound;
 };
 
 template <int N>

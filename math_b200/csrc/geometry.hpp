@@ -15,10 +15,12 @@
 
 // The overlap test is also compiled for the device (the GPU tree build): same operations, same order,
 // no contraction, so the device decides every box-simplex pair as the host does.
+#ifndef NT_HD
 #ifdef __CUDACC__
 #define NT_HD __host__ __device__
 #else
 #define NT_HD
+#endif
 #endif
 
 namespace ntrace

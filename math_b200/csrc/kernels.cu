@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(BLOCK) k_trace_closest(__grid_constant__ const
 {
         const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
         WalkStats ws{0, 0, 0, 0, 0};
+        const float* const bounds = walk_bounds<N>(M);
         // one ray per lane; the warp walks until all its lanes are done (no early exit: the leaf
         // step is warp-cooperative)
         bool walking = false;
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(BLOCK) k_trace_closest(__grid_constant__ const
                 float first, second;
                 if (root_slabs<N>(M, r.org, r.dir, &first, &second))
                 {
-                        walk_begin<N>(w, r, (first > 0) ? first : second, FLT_MAX);
+                        walk_begin<N>(M, w, r, (first > 0) ? first : second, FLT_MAX);
                         w.raw = i;
                         walking = true;
                 }
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(BLOCK) k_trace_closest(__grid_constant__ const
         {
                 float t = 0;
                 int f = -1;
-                const int status = walk_step_warp<N>(M, w, walking, retest, org, dir, &t, &f, &ws);
+                const int status = walk_step_warp<N>(M, bounds, w, walking, retest, org, dir, &t, &f, &ws);
                 if (walking && status != W_RUNNING)
                 {
                         walking = false;
@@ -855,6 +856,7 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
 {
         const long long count = (long long)counters[C_WALK_EXT];
         const MeshDev<N>& M = S.mesh[0];
+        const float* const bounds = walk_bounds<N>(M);
         WalkStats ws{0, 0, 0, 0, 0};
         long long rays = 0;
         long long i = -1;
@@ -880,7 +882,7 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
                                         r.dir[k] = A.at(N + k, j);
                                 }
                                 plan = plans[q];  // listed rays have plan.walk set
-                                walk_begin<N>(w, r, plan.mesh_t, FLT_MAX);
+                                walk_begin<N>(M, w, r, plan.mesh_t, FLT_MAX);
                                 i = j;
                         }
                         if (exhausted || !__any_sync(0xffffffffu, i < 0))
@@ -899,7 +901,7 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
                 {
                         float t = 0;
                         int f = -1;
-                        int status = walk_step_warp<N, R>(M, w, i >= 0, S.retest, nullptr, nullptr, &t, &f, &ws, S.walk_small);
+                        int status = walk_step_warp<N, R>(M, bounds, w, i >= 0, S.retest, nullptr, nullptr, &t, &f, &ws, S.walk_small);
                         if (i >= 0 && status != W_RUNNING)
                         {
                                 float tt;
@@ -930,6 +932,7 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
 {
         const long long count = (long long)counters[C_SHADOW];
         const MeshDev<N>& M = S.mesh[0];
+        const float* const bounds = walk_bounds<N>(M);
         WalkStats ws{0, 0, 0, 0, 0};
         long long rays = 0;
         long long i = -1;
@@ -955,7 +958,7 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
                                 // queued by k_shade: nothing nearer than the light occludes it, and the mesh's
                                 // root box starts before the light at the stored entry distance
                                 const float dj = SQ.at(2 * N, j);
-                                walk_begin<N>(w, r, SQ.at(2 * N + 4, j), dj);
+                                walk_begin<N>(M, w, r, SQ.at(2 * N + 4, j), dj);
                                 dist = dj;
                                 i = j;
                         }
@@ -975,7 +978,7 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
                 {
                         float t = 0;
                         int f = -1;
-                        int status = walk_step_warp<N, R>(M, w, i >= 0, S.retest, nullptr, nullptr, &t, &f, &ws, S.walk_small);
+                        int status = walk_step_warp<N, R>(M, bounds, w, i >= 0, S.retest, nullptr, nullptr, &t, &f, &ws, S.walk_small);
                         if (i >= 0 && status != W_RUNNING)
                         {
                                 if (!(status == W_HIT && t < dist))

@@ -6,6 +6,7 @@
 #include "geometry.hpp"
 #include "kernels.h"
 #include "treebuild.h"
+#include "walk_math.hpp"
 
 #include <algorithm>
 #include <atomic>
@@ -230,6 +231,9 @@ struct MeshHost
         std::vector<int32_t> leaf_idx;
         std::vector<float> level_sizes;  // (levels) x n
         std::vector<float> root_org, root_d1;
+        std::vector<float> bounds;  // the finest boxes' boundaries along each axis (MeshDev::bounds)
+        std::vector<float> inv_cell;
+        float near_bound = 0;
         float dist = 0;
         std::vector<float> vmin, vmax;
         long long leaf_count = 0;
@@ -237,6 +241,7 @@ struct MeshHost
         double build_seconds = 0;
         std::vector<int32_t> ntype;  // per facet: NormalType and reversed-vertex bits (MeshDev::ntype)
         DevBuf d_rec32, d_rec64, d_nodes, d_idx;
+        DevBuf d_bounds;
         DevBuf d_leafrec;  // rec32 gathered in leaf-list order (made on the device from d_rec32, d_idx)
         DevBuf d_normals, d_fnormals, d_ntype;
         // device staging copy of the four arrays (nt_scene_upload_begin / _commit)
@@ -257,9 +262,9 @@ struct MeshHost
                   normals(std::move(o.normals)), facet_normals(std::move(o.facet_normals)), rec32(std::move(o.rec32)),
                   rec64(std::move(o.rec64)), nodes(std::move(o.nodes)), leaf_idx(std::move(o.leaf_idx)),
                   level_sizes(std::move(o.level_sizes)), root_org(std::move(o.root_org)), root_d1(std::move(o.root_d1)),
-                  dist(o.dist), vmin(std::move(o.vmin)), vmax(std::move(o.vmax)), leaf_count(o.leaf_count),
+                  bounds(std::move(o.bounds)), inv_cell(std::move(o.inv_cell)), near_bound(o.near_bound), dist(o.dist), vmin(std::move(o.vmin)), vmax(std::move(o.vmax)), leaf_count(o.leaf_count),
                   degenerate(o.degenerate), build_seconds(o.build_seconds), ntype(std::move(o.ntype)),
-                  d_rec32(std::move(o.d_rec32)), d_rec64(std::move(o.d_rec64)), d_nodes(std::move(o.d_nodes)),
+                  d_bounds(std::move(o.d_bounds)), d_rec32(std::move(o.d_rec32)), d_rec64(std::move(o.d_rec64)), d_nodes(std::move(o.d_nodes)),
                   d_idx(std::move(o.d_idx)), d_leafrec(std::move(o.d_leafrec)), d_normals(std::move(o.d_normals)),
                   d_fnormals(std::move(o.d_fnormals)),
                   d_ntype(std::move(o.d_ntype)), d_stage(std::move(o.d_stage)),
@@ -671,6 +676,8 @@ void build_mesh(MeshHost& m, unsigned threads, bool tree_on_gpu, cudaStream_t st
                 }
         }
 
+        build_bounds<N>(m.root_org.data(), m.root_d1.data(), m.level_sizes, &m.bounds, &m.inv_cell, &m.near_bound);
+
         if (tree_on_gpu)
         {
                 TreeResult tr;
@@ -1003,6 +1010,12 @@ MeshDev<N> mesh_dev(const MeshHost& m)
                 }
         }
         d.dist = m.dist;
+        d.bounds = m.d_bounds.as<float>();
+        for (int k = 0; k < N; ++k)
+        {
+                d.inv_cell[k] = m.inv_cell[k];
+        }
+        d.near_bound = m.near_bound;
         return d;
 }
 
@@ -1061,6 +1074,7 @@ void build_scene(nt_scene* s, unsigned threads, bool host_only, bool tree_on_gpu
                         m.d_rec64.upload(m.rec64, s->stream);
                         m.d_nodes.upload(m.nodes, s->stream);
                         m.d_idx.upload(m.leaf_idx, s->stream);
+                        m.d_bounds.upload(m.bounds, s->stream);
                         gather_leaf_records(m, N, s->stream, s->leaf_records);
                         if (!m.ntype.empty())
                         {

@@ -1,0 +1,275 @@
+// Host check of the walk's shared arithmetic (math_b200/csrc/walk_math.hpp): the finest-cell index against
+// the descent it replaces, and the exit by approximate quotients against the exact slabs, for points on,
+// beside and between the box boundaries.  Prints one line per dimension; exits 1 on a difference.
+#include "walk_math.hpp"
+
+#include <array>
+#include <cstdio>
+#include <random>
+
+using namespace ntrace;
+
+namespace
+{
+// reciprocals off by up to 2^-22 either way, as an approximate unit's may be
+struct LooseQuotient
+{
+        static inline int turn = 0;
+        static float rcp(float x)
+        {
+                const float r = 1.0f / x;
+                return r * (1.0f + (float)((turn++ % 3) - 1) * 2.4e-7f);
+        }
+        static float div(float a, float b)
+        {
+                return a / b;
+        }
+};
+
+template <int N>
+struct Tree
+{
+        std::array<float, N> org, d1;
+        std::vector<float> sizes, bounds, inv_cell;
+        float near_bound, dist;
+};
+
+template <int N>
+Tree<N> make_tree(std::mt19937& rng)
+{
+        constexpr int LEVELS = TreeBits<N>::D + 2;
+        std::uniform_real_distribution<float> u(-3.0f, 3.0f);
+        Tree<N> t;
+        t.sizes.resize(LEVELS * N);
+        float all = 0;
+        for (int k = 0; k < N; ++k)
+        {
+                const float a = u(rng), b = u(rng);
+                t.org[k] = std::min(a, b) - 0.1f;
+                t.sizes[k] = std::max(a, b) + 0.1f - t.org[k];
+                t.d1[k] = t.org[k] + t.sizes[k];
+                all = std::max(all, std::max(std::fabs(t.org[k]), std::fabs(t.d1[k])));
+                for (int l = 1; l < LEVELS; ++l)
+                {
+                        t.sizes[l * N + k] = t.sizes[(l - 1) * N + k] / 2;
+                }
+        }
+        t.dist = all * (20 * std::numeric_limits<float>::epsilon());
+        build_bounds<N>(t.org.data(), t.d1.data(), t.sizes, &t.bounds, &t.inv_cell, &t.near_bound);
+        return t;
+}
+
+// the descent to the finest level: 0 found (code, org), 1 outside the root, 2 ambiguous or in a gap
+template <int N>
+int descend(const Tree<N>& t, const float* p, unsigned* code, float* o)
+{
+        bool ambiguous = false;
+        for (int k = 0; k < N; ++k)
+        {
+                if (!(p[k] <= t.d1[k]) || !(-p[k] <= -t.org[k]))
+                {
+                        return 1;
+                }
+                o[k] = t.org[k];
+        }
+        *code = 0;
+        for (int l = 0; l < TreeBits<N>::D; ++l)
+        {
+                for (int k = 0; k < N; ++k)
+                {
+                        const float h = t.sizes[(l + 1) * N + k];
+                        const float mid = o[k] + h;
+                        const bool lo = p[k] <= mid, hi = -p[k] <= -mid && p[k] <= mid + h;
+                        if (!lo && !hi)
+                        {
+                                return 2;
+                        }
+                        ambiguous |= lo && hi;
+                        if (!lo)
+                        {
+                                *code |= 1u << (k * TreeBits<N>::D + TreeBits<N>::D - 1 - l);
+                                o[k] = mid;
+                        }
+                }
+        }
+        return ambiguous ? 2 : 0;
+}
+
+// box_slabs and the nearest face (device.cuh's leaf_exit_exact) on the host
+template <int N>
+Exit<N> exact_exit(const float* org, const float* size, const float* cur, const float* dir)
+{
+        Exit<N> x{};
+        float f_max = -FLT_MAX, b_min = FLT_MAX;
+        for (int i = 0; i < N; ++i)
+        {
+                const float d1 = org[i] + size[i], d2 = -org[i], s = dir[i], d = cur[i];
+                if (s == 0)
+                {
+                        if (d - d1 > 0 || -d - d2 > 0)
+                        {
+                                return x;
+                        }
+                        continue;
+                }
+                const float a1 = (d1 - d) / s, a2 = (d2 + d) / -s;
+                b_min = std::min(b_min, s < 0 ? a2 : a1);
+                f_max = std::max(f_max, s < 0 ? a1 : a2);
+                if (b_min <= 0 || b_min < f_max)
+                {
+                        return x;
+                }
+        }
+        x.ok = true;
+        x.t = b_min;
+        float mn = FLT_MAX;
+        for (int i = 0; i < N; ++i)
+        {
+                x.ip[i] = cur[i] + dir[i] * b_min;
+                const float d1 = org[i] + size[i];
+                const float lh = std::fabs(x.ip[i] - d1), ll = std::fabs(x.ip[i] + (-org[i]));
+                if (lh < mn)
+                {
+                        mn = lh;
+                        x.nudge = i + 1;
+                }
+                if (ll < mn)
+                {
+                        mn = ll;
+                        x.nudge = -(i + 1);
+                }
+        }
+        return x;
+}
+
+template <int N>
+bool check(int trees, int points)
+{
+        constexpr int D = TreeBits<N>::D, CELLS = TreeBits<N>::CELLS;
+        std::mt19937 rng(17 + N);
+        std::uniform_real_distribution<float> u(0.0f, 1.0f);
+        std::normal_distribution<float> gauss;
+        long located = 0, left = 0, exits = 0, unsure = 0, ends = 0;
+        for (int it = 0; it < trees; ++it)
+        {
+                const Tree<N> t = make_tree<N>(rng);
+                for (int ip = 0; ip < points; ++ip)
+                {
+                        float p[N], o[N];
+                        for (int k = 0; k < N; ++k)
+                        {
+                                const float* b = t.bounds.data() + k * (CELLS + 1);
+                                const int pick = (int)(u(rng) * 30);
+                                p[k] = t.org[k] + (1.02f * u(rng) - 0.01f) * t.sizes[k];
+                                const float at = b[(int)(u(rng) * (CELLS + 0.999f))];
+                                // on a boundary, a few units in the last place beside one, nudged off one
+                                if (pick == 0)
+                                {
+                                        p[k] = at;
+                                }
+                                else if (pick == 1)
+                                {
+                                        p[k] = std::nextafter(at, u(rng) < 0.5f ? -9.0f : 9.0f);
+                                }
+                                else if (pick == 2)
+                                {
+                                        p[k] = at + (float)((int)(u(rng) * 9) - 4) * 1.2e-7f;
+                                }
+                                else if (pick == 3)
+                                {
+                                        p[k] = at + (u(rng) < 0.5f ? -t.dist : t.dist);
+                                }
+                        }
+                        unsigned code = 0, want = 0;
+                        const CellResult r = point_cell<N>(t.bounds.data(), t.org.data(), t.inv_cell.data(), t.near_bound, p, &code);
+                        const int e = descend<N>(t, p, &want, o);
+                        if (r != CELL_NEAR)
+                        {
+                                ++located;
+                                if ((r == CELL_OUTSIDE) != (e == 1) || (r == CELL_IN && (e != 0 || code != want)))
+                                {
+                                        std::printf("n=%d: cell of a point differs from its descent's\n", N);
+                                        return false;
+                                }
+                        }
+                        else
+                        {
+                                ++left;
+                        }
+                        if (e != 0)
+                        {
+                                continue;
+                        }
+                        // the children along the path, the level at which two cells' paths part
+                        const int level = (int)(u(rng) * (D + 0.999f));
+                        const unsigned other = want ^ (level < D ? 1u << ((ip % N) * D + D - 1 - level) : 0u);
+                        int part = 0;
+                        while (part < D && child_bits<N>(want, D - 1 - part) == child_bits<N>(other, D - 1 - part))
+                        {
+                                ++part;
+                        }
+                        const unsigned diff = cell_difference<N>(want, other);
+                        if (part != level || D - (diff ? 32 - __builtin_clz(diff) : 0) != level)
+                        {
+                                std::printf("n=%d: two cells' paths part at another level\n", N);
+                                return false;
+                        }
+                        // the exit from the box of a level, from inside it, from a face or from just outside
+                        float org[N], size[N], cur[N], dir[N], len = 0;
+                        for (int k = 0; k < N; ++k)
+                        {
+                                const unsigned c = ((want >> (k * D)) & (CELLS - 1)) >> (D - level) << (D - level);
+                                org[k] = t.bounds[k * (CELLS + 1) + c];
+                                size[k] = t.sizes[level * N + k];
+                                const int pick = (int)(u(rng) * 8);
+                                cur[k] = pick == 0 ? org[k] : (pick == 1 ? org[k] + size[k] : org[k] + u(rng) * size[k]);
+                                if (pick == 2)
+                                {
+                                        cur[k] = std::nextafter(u(rng) < 0.5f ? org[k] : org[k] + size[k], u(rng) < 0.5f ? -9.0f : 9.0f);
+                                }
+                                dir[k] = gauss(rng);
+                                const int zero = (int)(u(rng) * 16);
+                                dir[k] = zero == 0 ? 0.0f : (zero == 1 ? dir[k] * 1e-30f : (zero == 2 ? 1.0f : dir[k]));
+                                len += dir[k] * dir[k];
+                        }
+                        if (!(len > 0))
+                        {
+                                continue;
+                        }
+                        for (int k = 0; k < N; ++k)
+                        {
+                                dir[k] /= std::sqrt(len);
+                        }
+                        Exit<N> x;
+                        if (!leaf_exit_fast<N, LooseQuotient>(org, size, cur, dir, &x))
+                        {
+                                ++unsure;
+                                continue;
+                        }
+                        const Exit<N> w = exact_exit<N>(org, size, cur, dir);
+                        ++exits;
+                        ends += !w.ok;
+                        bool same = x.ok == w.ok;
+                        for (int k = 0; same && w.ok && k < N; ++k)
+                        {
+                                same = x.ip[k] == w.ip[k];
+                        }
+                        if (!same || (w.ok && (x.t != w.t || x.nudge != w.nudge)))
+                        {
+                                std::printf("n=%d: exit differs: t %g %g, face %d %d\n", N, x.t, w.t, x.nudge, w.nudge);
+                                return false;
+                        }
+                }
+        }
+        std::printf("n=%d: %ld located, %ld left to the descent; %ld exits (%ld of them ends), %ld left to the slabs\n", N,
+                    located, left, exits, ends, unsure);
+        // both rules must decide most cases, or the test shows nothing
+        return located > left / 2 && exits > unsure;
+}
+}
+
+int main(int argc, char** argv)
+{
+        const int points = argc > 1 ? std::atoi(argv[1]) : 2000;
+        return check<3>(60, points) && check<4>(60, points) && check<5>(60, points) && check<6>(60, points) ? 0 : 1;
+}
