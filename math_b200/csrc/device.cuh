@@ -9,10 +9,6 @@
 #include <cfloat>
 #include <cstdint>
 
-#ifndef NT_FACET_FULL_LOAD
-#define NT_FACET_FULL_LOAD 1
-#endif
-
 namespace ntrace
 {
 // ------------------------------------------------------------------------------------------------
@@ -267,7 +263,7 @@ struct Leaf
 {
         int node;  // -1: no leaf contains the point
         int level;
-        float org[N];
+        unsigned code;  // the indices of its first finest cell along the axes (point_cell)
 };
 
 template <int N>
@@ -275,6 +271,14 @@ struct Point
 {
         float v[N];
 };
+
+// The cell-index bit of axis i that the half taken below `level` sets.
+template <int N>
+__device__ __forceinline__ unsigned level_bit(int i, int level, int half)
+{
+        const int bit = TreeBits<N>::D - 1 - level;
+        return bit >= 0 ? (unsigned)half << (i * TreeBits<N>::D + bit) : 0u;
+}
 
 // Out of line and by value: the caller's walk state is not address-taken, so it stays in registers.
 template <int N>
@@ -284,22 +288,19 @@ __device__ __noinline__ Leaf<N> find_leaf_dfs(const MeshDev<N>& M, const Point<N
         Leaf<N> res;
         res.node = -1;
         res.level = 0;
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-        {
-                res.org[i] = 0;
-        }
-        Leaf<N>* out = &res;
+        res.code = 0;
         struct Frame
         {
                 int node;
                 int next;
+                unsigned code;
                 float org[N];
         };
         Frame st[MAX_LEVELS + 1];
         int top = 0;
         st[0].node = 0;
         st[0].next = 0;
+        st[0].code = 0;
 #pragma unroll
         for (int i = 0; i < N; ++i)
         {
@@ -311,12 +312,9 @@ __device__ __noinline__ Leaf<N> find_leaf_dfs(const MeshDev<N>& M, const Point<N
                 int2 nd = M.nodes[f.node];
                 if (nd.y >= 0)
                 {
-                        out->node = f.node;
-                        out->level = top;
-                        for (int i = 0; i < N; ++i)
-                        {
-                                out->org[i] = f.org[i];
-                        }
+                        res.node = f.node;
+                        res.level = top;
+                        res.code = f.code;
                         return res;
                 }
                 bool pushed = false;
@@ -340,9 +338,11 @@ __device__ __noinline__ Leaf<N> find_leaf_dfs(const MeshDev<N>& M, const Point<N
                                 Frame& g = st[top + 1];
                                 g.node = nd.x + c;
                                 g.next = 0;
+                                g.code = f.code;
                                 for (int i = 0; i < N; ++i)
                                 {
                                         g.org[i] = co[i];
+                                        g.code |= level_bit<N>(i, top, (c >> i) & 1);
                                 }
                                 ++top;
                                 pushed = true;
@@ -372,15 +372,17 @@ constexpr int WALK_BLOCK = NT_BLOCK;
 // new point shares the path down to the first level at which an index bit differs, so its descent
 // starts there: the first child of the internal node at each level of the path is kept in shared memory
 // (path_cache_slots).
+constexpr int PATH_COLD = 0x100;
+
 struct PathCache
 {
-        int depth;      // level of the cached leaf; -1: empty
+        int depth;      // level of the cached leaf; PATH_COLD set: the path above it is not in the slots
         int2 leaf;      // the cached leaf's record
         unsigned code;  // the cell indices, axis i at bit i x D
 
         __device__ __forceinline__ void reset()
         {
-                depth = -1;
+                depth = PATH_COLD;
                 leaf = make_int2(0, 0);
                 code = 0;
         }
@@ -425,6 +427,7 @@ __device__ __noinline__ Located<N> locate_exact(const MeshDev<N>& M, const Point
         Located<N> res;
         res.leaf.node = -1;
         res.leaf.level = 0;
+        res.leaf.code = 0;
         res.rec = make_int2(0, 0);
         res.levels = 0;
         float o[N];
@@ -433,7 +436,6 @@ __device__ __noinline__ Located<N> locate_exact(const MeshDev<N>& M, const Point
         for (int i = 0; i < N; ++i)
         {
                 o[i] = M.root_org[i];
-                res.leaf.org[i] = 0;
                 outside |= !(pt.v[i] <= M.root_d1[i]) || !(-pt.v[i] <= -M.root_org[i]);
         }
         if (outside)
@@ -441,6 +443,7 @@ __device__ __noinline__ Located<N> locate_exact(const MeshDev<N>& M, const Point
                 return res;
         }
         int node = 0;
+        unsigned code = 0;
         bool ambiguous = false;
         for (int lvl = 0; lvl < MAX_LEVELS; ++lvl)
         {
@@ -450,11 +453,7 @@ __device__ __noinline__ Located<N> locate_exact(const MeshDev<N>& M, const Point
                 {
                         res.leaf.node = node;
                         res.leaf.level = lvl;
-#pragma unroll
-                        for (int i = 0; i < N; ++i)
-                        {
-                                res.leaf.org[i] = o[i];
-                        }
+                        res.leaf.code = code;
                         res.rec = nd;
                         return res;
                 }
@@ -474,6 +473,7 @@ __device__ __noinline__ Located<N> locate_exact(const MeshDev<N>& M, const Point
                         else if (hi_ok)
                         {
                                 child |= 1 << i;
+                                code |= level_bit<N>(i, lvl, 1);
                                 o[i] = mid;
                         }
                         else
@@ -498,16 +498,16 @@ __device__ __noinline__ Located<N> locate_exact(const MeshDev<N>& M, const Point
         return res;
 }
 
-// The leaf that contains p (find_box_for_point, tree.h:441-463): the path to it is the bits of its finest
-// cell (point_cell, `bounds` the mesh's table in shared or global memory), and nodes are read only from
-// the first level at which that path leaves the cached one.  Points at a box boundary take the exact
-// descent.  *descent counts the levels of the full descent, which is the algorithm's work.
+// The leaf that contains p (find_box_for_point, tree.h:441-463), left in the path cache: the path to it
+// is the bits of p's finest cell (point_cell, `bounds` the mesh's table in shared or global memory), and
+// nodes are read only from the first level at which that path leaves the cached one.  Points at a box
+// boundary take the exact descent.  *descent counts the levels of the full descent, which is the
+// algorithm's work.
 template <int N>
 __device__ __forceinline__ bool locate_leaf(const MeshDev<N>& M, const float* bounds, const float* p, PathCache& pc,
-                                            Leaf<N>* out, int2* leaf_rec, unsigned* descent)
+                                            unsigned* descent)
 {
         constexpr int D = TreeBits<N>::D;
-        constexpr int CELLS = TreeBits<N>::CELLS;
         unsigned code;
         const CellResult cell = point_cell<N>(bounds, M.root_org, M.inv_cell, M.near_bound, p, &code);
         if (cell == CELL_NEAR)
@@ -520,8 +520,9 @@ __device__ __forceinline__ bool locate_leaf(const MeshDev<N>& M, const float* bo
                 }
                 const Located<N> r = locate_exact<N>(M, pt);
                 *descent += r.levels;
-                *out = r.leaf;
-                *leaf_rec = r.rec;
+                pc.depth = r.leaf.level | PATH_COLD;
+                pc.leaf = r.rec;
+                pc.code = r.leaf.code;
                 return r.leaf.node >= 0;
         }
         if (cell == CELL_OUTSIDE)
@@ -534,23 +535,17 @@ __device__ __forceinline__ bool locate_leaf(const MeshDev<N>& M, const float* bo
         int2 nd = pc.leaf;
         if (lvl >= pc.depth)
         {
-                if (pc.depth < 0)
-                {
-                        nd = __ldg(&M.nodes[0]);
-                        lvl = 0;
-                        if (nd.y < 0)
-                        {
-                                fc[0] = nd.x;
-                        }
-                }
-                else
-                {
-                        lvl = pc.depth;
-                }
+                lvl = pc.depth;
+        }
+        else if (pc.depth < PATH_COLD)
+        {
+                nd = make_int2(fc[lvl * WALK_BLOCK], -1);
         }
         else
         {
-                nd = make_int2(fc[lvl * WALK_BLOCK], -1);
+                lvl = 0;
+                nd = __ldg(&M.nodes[0]);
+                fc[0] = nd.x;
         }
         while (nd.y < 0)
         {
@@ -561,7 +556,7 @@ __device__ __forceinline__ bool locate_leaf(const MeshDev<N>& M, const float* bo
                         if (lvl >= D)
                         {
                                 // deeper than the depth limit: not a tree this library builds
-                                pc.depth = -1;
+                                pc.depth = PATH_COLD;
                                 return false;
                         }
                         fc[lvl * WALK_BLOCK] = nd.x;
@@ -570,17 +565,28 @@ __device__ __forceinline__ bool locate_leaf(const MeshDev<N>& M, const float* bo
         pc.code = code;
         pc.depth = lvl;
         pc.leaf = nd;
-        *leaf_rec = nd;
         *descent += lvl + 1;
-        out->node = 0;
-        out->level = lvl;
+        return true;
+}
+
+// The origin and size of the leaf in the path cache.  The origin is the boundary at its first finest
+// cell; the size is the root's halved per level (exact), without an indexed read of the parameters that
+// differs from lane to lane.
+template <int N>
+__device__ __forceinline__ void leaf_box(const MeshDev<N>& M, const float* bounds, const PathCache& pc, float* org,
+                                         float* size)
+{
+        constexpr int D = TreeBits<N>::D;
+        constexpr int CELLS = TreeBits<N>::CELLS;
+        const int level = pc.depth & (PATH_COLD - 1);
+        const float scale = __int_as_float((127 - level) << 23);
+        const unsigned keep = (CELLS - 1) & ~((1u << (D - level)) - 1);
 #pragma unroll
         for (int i = 0; i < N; ++i)
         {
-                const unsigned c = (code >> (i * D)) & (CELLS - 1);
-                out->org[i] = bounds[i * (CELLS + 1) + ((c >> (D - lvl)) << (D - lvl))];
+                org[i] = bounds[i * (CELLS + 1) + ((pc.code >> (i * D)) & keep)];
+                size[i] = M.size[0][i] * scale;
         }
-        return true;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -651,19 +657,6 @@ __device__ __forceinline__ Exit<N> leaf_exit(const float* org, const float* size
         return x;
 }
 
-// The size of the boxes at a level: the root's halved per level (exact), without an indexed read of the
-// parameters that differs from lane to lane.
-template <int N>
-__device__ __forceinline__ void level_size(const MeshDev<N>& M, int level, float* size)
-{
-        const float scale = __int_as_float((127 - level) << 23);
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-        {
-                size[i] = M.size[0][i] * scale;
-        }
-}
-
 // ------------------------------------------------------------------------------------------------
 // Ray versus (N-1)-simplex.
 //
@@ -678,25 +671,21 @@ enum TestResult : int
         T_UNSURE = 2
 };
 
-// STAGED: the record lies in shared memory (staged by cp.async, leaf_closest_warp) and is read with
-// plain loads; otherwise it is read from global memory through the read-only path.
-template <int N, bool STAGED = false>
+// STRIDE > 0: the record lies in shared memory, its 16-byte words STRIDE words apart (pool_stage), each
+// read where it is needed; otherwise it is read from global memory through the read-only path.
+template <int N, int STRIDE = 0>
 __device__ __forceinline__ int facet_test32(const float4* rec, const Ray<N>& r, float ao, float* t_out)
 {
         constexpr float EPS = 5.9604645e-08f;  // 2^-24
-        // the whole record is read at once (one memory round trip; measured faster than reading each
-        // barycentric plane only once the tests before it have passed, NT_FACET_FULL_LOAD=0, which
-        // saves bytes but waits up to N times)
-#if NT_FACET_FULL_LOAD
-        constexpr int HEAD4 = Rec32<N>::F4;
-#else
-        constexpr int HEAD4 = (Rec32<N>::OFF_PLANES + 3) / 4;
-#endif
+        constexpr bool STAGED = STRIDE > 0;
+        // from global memory the whole record is read at once: one round trip (measured faster than reading
+        // each barycentric plane only once the tests before it have passed)
+        constexpr int HEAD4 = STAGED ? (Rec32<N>::OFF_PLANES + 3) / 4 : Rec32<N>::F4;
         float f[Rec32<N>::FLOATS];
 #pragma unroll
         for (int q = 0; q < HEAD4; ++q)
         {
-                float4 v = STAGED ? rec[q] : __ldg(rec + q);
+                float4 v = STAGED ? rec[q * STRIDE] : __ldg(rec + q);
                 f[4 * q + 0] = v.x;
                 f[4 * q + 1] = v.y;
                 f[4 * q + 2] = v.z;
@@ -744,7 +733,7 @@ __device__ __forceinline__ int facet_test32(const float4* rec, const Ray<N>& r, 
 #pragma unroll
                 for (int q = first4; q < need4; ++q)
                 {
-                        float4 v = STAGED ? rec[q] : __ldg(rec + q);
+                        float4 v = STAGED ? rec[q * STRIDE] : __ldg(rec + q);
                         f[4 * q + 0] = v.x;
                         f[4 * q + 1] = v.y;
                         f[4 * q + 2] = v.z;
@@ -1040,13 +1029,12 @@ __device__ bool mesh_closest(const MeshDev<N>& M, const Ray<N>& ray, float root_
         // the bound leaves ample margin and turns a walk that does not advance into an error flag
         for (int step = 0; step < 16384; ++step)
         {
-                Leaf<N> lf;
-                int2 nd;
-                if (locate_leaf<N>(M, M.bounds, probe, pc, &lf, &nd, &ws->descent))
+                if (locate_leaf<N>(M, M.bounds, probe, pc, &ws->descent))
                 {
                         ++ws->box_steps;
-                        float sz[N];
-                        level_size<N>(M, lf.level, sz);
+                        const int2 nd = pc.leaf;
+                        float org[N], sz[N];
+                        leaf_box<N>(M, M.bounds, pc, org, sz);
                         if (travelled > tmax * 1.00001f + 1e-6f)
                         {
                                 return false;
@@ -1063,8 +1051,8 @@ __device__ bool mesh_closest(const MeshDev<N>& M, const Ray<N>& ray, float root_
 #pragma unroll
                                         for (int i = 0; i < N; ++i)
                                         {
-                                                float d1 = lf.org[i] + sz[i];
-                                                if (!(pt[i] <= d1) || !(-pt[i] <= -lf.org[i]))
+                                                float d1 = org[i] + sz[i];
+                                                if (!(pt[i] <= d1) || !(-pt[i] <= -org[i]))
                                                 {
                                                         inside = false;
                                                 }
@@ -1077,7 +1065,7 @@ __device__ bool mesh_closest(const MeshDev<N>& M, const Ray<N>& ray, float root_
                                         }
                                 }
                         }
-                        const Exit<N> ex = leaf_exit<N>(lf.org, sz, cur, ray.dir);
+                        const Exit<N> ex = leaf_exit<N>(org, sz, cur, ray.dir);
                         if (!ex.ok)
                         {
                                 return false;
@@ -1364,7 +1352,7 @@ __device__ bool scene_visible(const DevScene<N>& S, const Ray<N>& r, float dist,
 // Resumable tree walk for scenes with exactly one mesh.
 //
 // The same walk as mesh_closest, cut at leaf granularity: each call of walk_step_warp visits one
-// leaf (descent, leaf facets, exit) and says whether the walk has ended.  A lane whose walk ends
+// leaf (location, exit, leaf facets) and says whether the walk has ended.  A lane whose walk ends
 // takes the next ray at once while the other lanes of its warp continue theirs, so warps stay full
 // even though rays visit very different numbers of leaves (the per-ray loop leaves most lanes idle).
 // The decisions around the walk are those of ray_intersection (ray_intersection.h:26-105) and
@@ -1468,54 +1456,44 @@ __device__ __forceinline__ void walk_begin(const MeshDev<N>& M, Walk<N>& w, cons
 // The leaves that the 32 lanes of a warp stand in hold different numbers of facets (0 to a few
 // dozen), so a per-lane loop over them leaves most lanes idle.  Here the warp pools its facet tests:
 // the lanes' facet lists are laid end to end (warp prefix sum of the counts) and every lane tests
-// every 32nd entry of the pooled list against the owning lane's ray, fetched by shuffle.  Each
-// outcome (FP32 hit, or hit after the FP64 re-test) goes to a per-warp shared-memory slot; the owner
-// then reads its own slots in leaf-list order and makes the same sequential choice as leaf_closest
-// (strict < in list order, near-ties settled in FP64), so the result is the per-lane loop's.
+// every 32nd entry of the pooled list against the owning lane's ray, fetched by shuffle.  The hits of a
+// round (FP32 hits, or hits after the FP64 re-test) are known to the whole warp by ballot and left in
+// shared memory; each owner reads its own ones in leaf-list order and makes the same sequential choice
+// as leaf_closest (strict < in list order, near-ties settled in FP64), so the result is the per-lane
+// loop's.  Most tests miss: reading the hits alone instead of every outcome, and working the exit out
+// before the tests, took the n = 4 frame (675,461 facets) from 29.6 to 27.0 ms, n = 3 from 2.88 to 2.49.
+// Making lanes with facets wait until 8, 16 or 24 of the warp's lanes have some measured slower (3 to
+// 14 %): most leaves on a ray's way hold facets.
 
-constexpr int POOL_SLOTS = 128;  // pooled tests per warp and round, at most
 constexpr int SMALL_LEAF = 2;  // default: leaves this small are tested per lane, not pooled
 
 struct PoolSlot
 {
         float t;      // FP32 distance (the rounded FP64 one after a re-test)
-        int facet;    // -1: missed
+        int facet;
         double t64;   // FP64 distance when re-tested; -1 otherwise
 };
 
-// The warp's outcome slots, SLOTS of them (a kernel variant's chunk size: 32 to POOL_SLOTS).
-template <int SLOTS>
+// The warp's outcome slots: one per lane, written only for tests that hit.
 __device__ __forceinline__ PoolSlot* warp_pool()
 {
-        __shared__ PoolSlot s_pool[(WALK_BLOCK / 32) * SLOTS];
-        return s_pool + (threadIdx.x >> 5) * SLOTS;
+        __shared__ PoolSlot s_pool[WALK_BLOCK];
+        return s_pool + (threadIdx.x & ~31);
 }
 
-// Facet records staged through shared memory.  A warp handles its pooled tests in chunks of
-// Stage<N>::SLOTS: it first reads the chunk's facet indices (ROUNDS independent loads per lane), then
-// copies their records into its staging slots with cp.async (ROUNDS x F4 16-byte copies per lane in
-// flight at once), waits once, and tests from shared memory.  A chunk costs two memory round trips
-// instead of two per 32 tests.  The buffer is dynamic shared memory (Stage<N>::BYTES per block of
-// WALK_BLOCK threads), at most 8 KB per warp.
-// Other chunk sizes (R = 1, 2 or 4 rounds) are compiled as kernel variants that the autotuner
-// chooses from (nt_render_opts.walk_chunk).
-template <int N>
-struct StageFit
-{
-        static constexpr int REC_BYTES = Rec32<N>::F4 * 16;
-        static constexpr int FIT = 8192 / (32 * REC_BYTES);
-        static constexpr int ROUNDS = FIT < 1 ? 1 : (FIT > 4 ? 4 : (FIT == 3 ? 2 : FIT));
-};
-
-// R = 0: no staging; the records are read straight from global memory, 32 tests per round.
-template <int N, int R = StageFit<N>::ROUNDS>
+// Facet records staged through shared memory: the pooled tests are handled in chunks of 32 x R; a chunk's
+// records are copied with cp.async (R x F4 16-byte copies per lane in flight at once) into the warp's
+// staging slots, 16-byte word q of slot k at q x SLOTS + k, so that the copies and the reads of a warp
+// meet no bank conflicts.  The first chunk's copies are started before the exit from the leaf is worked
+// out and waited for after it.  R = 0: no staging; the records are read straight from global memory.
+// R = 1, 2 and 4 are kernel variants that the autotuner chooses from (nt_render_opts.walk_chunk).
+template <int N, int R>
 struct Stage
 {
         static constexpr int REC_BYTES = Rec32<N>::F4 * 16;
         static constexpr int ROUNDS = R > 0 ? R : 1;
         static constexpr int SLOTS = 32 * ROUNDS;
         static constexpr int BYTES = R > 0 ? (WALK_BLOCK / 32) * SLOTS * REC_BYTES : 0;
-        static_assert(SLOTS <= POOL_SLOTS, "a chunk's outcomes must fit the warp's pool");
 };
 
 __device__ __forceinline__ float4* stage_base()
@@ -1536,23 +1514,80 @@ __device__ __forceinline__ void cp_async_wait_all()
         asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// Closest facet of this lane's leaf (facets leaf_idx[start .. start + cnt)); every lane of the warp
-// calls it, lanes without a leaf with cnt = 0.  raw_org/raw_dir: the caller's raw rays for the
-// FP64 re-test of the fixed-ray-set query (null when rendering: the FP32 ray is promoted).
-template <int N, int RR = StageFit<N>::ROUNDS>
-__device__ __forceinline__ int leaf_closest_warp(const MeshDev<N>& M, int start, int cnt, const Ray<N>& ray, float ao,
-                                                 long long raw, const float* raw_org, const float* raw_dir, int retest,
-                                                 float* t_best, WalkStats* ws, int small_leaf = SMALL_LEAF)
+// The warp's pooled list of facet tests: the lanes' leaf lists laid end to end.
+struct WarpPool
+{
+        int start, cnt;  // this lane's leaf list
+        int excl;        // where it starts in the pooled list
+        int total;       // the pooled list's length; 0: nothing pooled
+};
+
+// Entry k of the pooled list: the lane that owns it and its position in the leaf lists.  Every lane of
+// the warp calls it.
+__device__ __forceinline__ int pool_entry(const WarpPool& P, int k, int* owner)
+{
+        const unsigned full = 0xffffffffu;
+        // owner: the last lane whose list starts at or before k
+        int o = 0;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+        {
+                const int v = __shfl_sync(full, P.excl, o + step);
+                if (v <= k)
+                {
+                        o += step;
+                }
+        }
+        *owner = o;
+        return __shfl_sync(full, P.start - P.excl, o) + k;
+}
+
+template <int N, int RR>
+__device__ __forceinline__ float4* warp_stage()
+{
+        return stage_base() + (size_t)(threadIdx.x >> 5) * Stage<N, RR>::SLOTS * Rec32<N>::F4;
+}
+
+// Copies the records of the pooled entries [cb, cb + SLOTS) into the warp's staging slots; own: their
+// owners (8 bits per round).
+template <int N, int RR>
+__device__ __forceinline__ void pool_stage(const MeshDev<N>& M, const WarpPool& P, int cb, int* pos, int* own)
+{
+        constexpr int R = Stage<N, RR>::ROUNDS;
+        constexpr int SLOTS = Stage<N, RR>::SLOTS;
+        float4* const stage = warp_stage<N, RR>();
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+        {
+                const int k = cb + 32 * r + (threadIdx.x & 31);
+                pos[r] = pool_entry(P, k, &own[r]);
+                if (RR > 0 && k < P.total)
+                {
+                        const float4* src = leaf_record<N>(M, pos[r]);
+#pragma unroll
+                        for (int q = 0; q < Rec32<N>::F4; ++q)
+                        {
+                                cp_async16(stage + q * SLOTS + 32 * r + (threadIdx.x & 31), src + q);
+                        }
+                }
+        }
+}
+
+// Pools the lanes' leaf lists and, staged, starts the copies of the first chunk's records (pos, own:
+// that chunk's entries).  Every lane of the warp calls it, lanes without a leaf with cnt = 0.  Small
+// leaves (at most small_leaf facets in every lane's leaf) are not pooled: P->total = 0.
+template <int N, int RR>
+__device__ __forceinline__ void pool_begin(const MeshDev<N>& M, int start, int cnt, int small_leaf, WarpPool* P, int* pos,
+                                           int* own)
 {
         const unsigned full = 0xffffffffu;
         const int lane = threadIdx.x & 31;
-        // small leaves (at most small_leaf facets in every lane's leaf, the common case: a walk step tests
-        // one or two facets on average) are tested by each lane on its own, in list order: the pooling's
-        // scan, owner search, shuffles and second pass would cost more than the idle lanes they save
+        P->start = start;
+        P->cnt = cnt;
+        P->total = 0;
         if ((int)__reduce_max_sync(full, (unsigned)cnt) <= small_leaf)
         {
-                return leaf_closest<N>(M, make_int2(start, cnt), ray, ao, Ray64Source<N>{raw_org, raw_dir, raw}, retest,
-                                       t_best, ws);
+                return;
         }
         int incl = cnt;
 #pragma unroll
@@ -1564,73 +1599,55 @@ __device__ __forceinline__ int leaf_closest_warp(const MeshDev<N>& M, int start,
                         incl += v;
                 }
         }
-        const int total = __shfl_sync(full, incl, 31);
-        const int excl = incl - cnt;
+        P->total = __shfl_sync(full, incl, 31);
+        P->excl = incl - cnt;
+        pool_stage<N, RR>(M, *P, 0, pos, own);
+}
+
+// Closest facet of this lane's leaf; every lane of the warp calls it after pool_begin.
+// raw_org/raw_dir: the caller's raw rays for the FP64 re-test of the fixed-ray-set query (null when
+// rendering: the FP32 ray is promoted).
+template <int N, int RR>
+__device__ __forceinline__ int pool_closest(const MeshDev<N>& M, const WarpPool& P, int* pos, int* own, const Ray<N>& ray,
+                                            float ao, long long raw, const float* raw_org, const float* raw_dir, int retest,
+                                            float* t_best, WalkStats* ws)
+{
+        const unsigned full = 0xffffffffu;
+        const int lane = threadIdx.x & 31;
+        const Ray64Source<N> own_src{raw_org, raw_dir, raw};
+        if (P.total == 0)
+        {
+                // the pooling's scan, owner search, shuffles and second pass would cost more than the idle
+                // lanes they save
+                return leaf_closest<N>(M, make_int2(P.start, P.cnt), ray, ao, own_src, retest, t_best, ws);
+        }
         int best = -1;
         float bt = FLT_MAX;
         double bt64 = 0;
         bool b64 = false;
-        if (total == 0)
-        {
-                *t_best = bt;
-                return best;
-        }
-        PoolSlot* pool = warp_pool<Stage<N, RR>::SLOTS>();
+        PoolSlot* pool = warp_pool();
         constexpr bool STAGED = RR > 0;
         constexpr int R = Stage<N, RR>::ROUNDS;
-        constexpr int F4 = Rec32<N>::F4;
-        float4* const stage = stage_base() + (size_t)(threadIdx.x >> 5) * Stage<N, RR>::SLOTS * F4;
-        const Ray64Source<N> own_src{raw_org, raw_dir, raw};
-        for (int cb = 0; cb < total; cb += Stage<N, RR>::SLOTS)
+        constexpr int SLOTS = Stage<N, RR>::SLOTS;
+        float4* const stage = warp_stage<N, RR>();
+        for (int cb = 0; cb < P.total; cb += SLOTS)
         {
-                const int ce = min(total, cb + Stage<N, RR>::SLOTS);
-                // the chunk's entries (positions in the leaf lists, whose records lie in that order in
-                // leaf_rec32), then, staged, their records into the staging slots (all copies in flight
-                // at once); a facet's index is read only for the tests that do not miss
-                int own[R];
-                int pos[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r)
+                if (cb > 0)
                 {
-                        const int k = cb + 32 * r + lane;
-                        // owner: the last lane whose list starts at or before k
-                        int o = 0;
-#pragma unroll
-                        for (int step = 16; step > 0; step >>= 1)
-                        {
-                                int v = __shfl_sync(full, excl, o + step);
-                                if (v <= k)
-                                {
-                                        o += step;
-                                }
-                        }
-                        own[r] = o;
-                        const int o_start = __shfl_sync(full, start, o);
-                        const int o_excl = __shfl_sync(full, excl, o);
-                        pos[r] = (k < ce) ? o_start + (k - o_excl) : -1;
+                        pool_stage<N, RR>(M, P, cb, pos, own);
                 }
-                if constexpr (STAGED)
+                if (STAGED)
                 {
-#pragma unroll
-                        for (int r = 0; r < R; ++r)
-                        {
-                                if (pos[r] >= 0)
-                                {
-                                        const float4* src = leaf_record<N>(M, pos[r]);
-                                        float4* dst = stage + (size_t)(32 * r + lane) * F4;
-#pragma unroll
-                                        for (int q = 0; q < F4; ++q)
-                                        {
-                                                cp_async16(dst + q, src + q);
-                                        }
-                                }
-                        }
                         cp_async_wait_all();
                 }
 #pragma unroll
                 for (int r = 0; r < R; ++r)
                 {
-                        const int k = cb + 32 * r + lane;
+                        const int base = cb + 32 * r;
+                        if (R > 1 && base >= P.total)
+                        {
+                                break;
+                        }
                         const int o = own[r];
                         const float o_ao = __shfl_sync(full, ao, o);
                         Ray<N> rr;
@@ -1641,142 +1658,135 @@ __device__ __forceinline__ int leaf_closest_warp(const MeshDev<N>& M, int start,
                                 rr.dir[i] = __shfl_sync(full, ray.dir[i], o);
                         }
                         const long long o_raw = raw_org ? __shfl_sync(full, raw, o) : 0;
-                        if (k < ce)
+                        bool keep = false;
+                        if (base + lane < P.total)
                         {
                                 ++ws->facet_tests;
                                 float t = -1.0f;
                                 double t64 = -1.0;
-                                int keep = -1;
-                                int res = STAGED ? facet_test32<N, true>(stage + (size_t)(32 * r + lane) * F4, rr, o_ao, &t)
-                                                 : facet_test32<N, false>(leaf_record<N>(M, pos[r]), rr, o_ao, &t);
-                                const int f = res != T_MISS ? __ldg(&M.leaf_idx[pos[r]]) : -1;
-                                if (res == T_HIT)
+                                int res = STAGED ? facet_test32<N, SLOTS>(stage + 32 * r + lane, rr, o_ao, &t)
+                                                 : facet_test32<N, 0>(leaf_record<N>(M, pos[r]), rr, o_ao, &t);
+                                if (res != T_MISS)
                                 {
-                                        keep = f;
-                                }
-                                else if (res == T_UNSURE)
-                                {
-                                        if (!retest)
+                                        const int f = __ldg(&M.leaf_idx[pos[r]]);
+                                        keep = true;
+                                        if (res == T_UNSURE)
                                         {
-                                                // without the re-test an uncertain FP32 hit counts when
-                                                // its distance is positive
-                                                if (t > 0)
+                                                if (!retest)
                                                 {
-                                                        keep = f;
-                                                }
-                                        }
-                                        else
-                                        {
-                                                ++ws->retests;
-                                                t64 = retest_facet<N>(M.rec64 + (size_t)f * Rec64<N>::DOUBLES, rr,
-                                                                      Ray64Source<N>{raw_org, raw_dir, o_raw});
-                                                if (t64 > 0)
-                                                {
-                                                        keep = f;
-                                                        t = (float)t64;
+                                                        // without the re-test an uncertain FP32 hit counts
+                                                        // when its distance is positive
+                                                        keep = t > 0;
                                                 }
                                                 else
                                                 {
-                                                        t64 = -1.0;
+                                                        ++ws->retests;
+                                                        t64 = retest_facet<N>(M.rec64 + (size_t)f * Rec64<N>::DOUBLES, rr,
+                                                                              Ray64Source<N>{raw_org, raw_dir, o_raw});
+                                                        keep = t64 > 0;
+                                                        t = (float)t64;
                                                 }
                                         }
+                                        PoolSlot& s = pool[lane];
+                                        s.t = t;
+                                        s.facet = f;
+                                        s.t64 = t64;
                                 }
-                                PoolSlot& s = pool[k - cb];
-                                s.t = t;
-                                s.facet = keep;
-                                s.t64 = t64;
                         }
-                }
-                __syncwarp();
-                // the owner's sequential choice over its slots of this round, in list order
-                const int q0 = max(excl, cb);
-                const int q1 = min(excl + cnt, ce);
-                for (int q = q0; q < q1; ++q)
-                {
-                        const PoolSlot s = pool[q - cb];
-                        if (s.facet < 0)
+                        const unsigned hits = __ballot_sync(full, keep);
+                        if (!hits)
                         {
                                 continue;
                         }
-                        const int f = s.facet;
-                        float t = s.t;
-                        double t64 = s.t64;
-                        bool is64 = t64 > 0;
-                        bool closer;
-                        float tol = 1e-5f * (fabsf(t) + ao) + 1e-30f;
-                        if (retest && best >= 0 && fabsf(t - bt) <= tol)
+                        __syncwarp();
+                        // the owner's sequential choice over its hits of this round, in list order
+                        const int q0 = min(max(P.excl - base, 0), 32);
+                        const int q1 = min(max(P.excl + P.cnt - base, 0), 32);
+                        unsigned mine = hits & (unsigned)((1ull << q1) - (1ull << q0));
+                        while (mine)
                         {
-                                if (!is64)
+                                const PoolSlot s = pool[__ffs(mine) - 1];
+                                mine &= mine - 1;
+                                const int f = s.facet;
+                                float t = s.t;
+                                double t64 = s.t64;
+                                bool is64 = t64 > 0;
+                                bool closer;
+                                float tol = 1e-5f * (fabsf(t) + ao) + 1e-30f;
+                                if (retest && best >= 0 && fabsf(t - bt) <= tol)
                                 {
-                                        ++ws->retests;
-                                        t64 = retest_facet<N>(M.rec64 + (size_t)f * Rec64<N>::DOUBLES, ray, own_src);
-                                        if (!(t64 > 0))
+                                        if (!is64)
                                         {
-                                                continue;
+                                                ++ws->retests;
+                                                t64 = retest_facet<N>(M.rec64 + (size_t)f * Rec64<N>::DOUBLES, ray, own_src);
+                                                if (!(t64 > 0))
+                                                {
+                                                        continue;
+                                                }
+                                                is64 = true;
                                         }
-                                        is64 = true;
+                                        if (!b64)
+                                        {
+                                                ++ws->retests;
+                                                double tb = retest_facet<N>(M.rec64 + (size_t)best * Rec64<N>::DOUBLES, ray,
+                                                                            own_src);
+                                                if (tb > 0)
+                                                {
+                                                        bt64 = tb;
+                                                        b64 = true;
+                                                }
+                                                else
+                                                {
+                                                        // the incumbent fails in FP64: the newcomer wins
+                                                        best = f;
+                                                        bt = (float)t64;
+                                                        bt64 = t64;
+                                                        b64 = true;
+                                                        continue;
+                                                }
+                                        }
+                                        closer = t64 < bt64;
                                 }
-                                if (!b64)
+                                else
                                 {
-                                        ++ws->retests;
-                                        double tb = retest_facet<N>(M.rec64 + (size_t)best * Rec64<N>::DOUBLES, ray, own_src);
-                                        if (tb > 0)
-                                        {
-                                                bt64 = tb;
-                                                b64 = true;
-                                        }
-                                        else
-                                        {
-                                                // the incumbent fails in FP64: the newcomer wins
-                                                best = f;
-                                                bt = (float)t64;
-                                                bt64 = t64;
-                                                b64 = true;
-                                                continue;
-                                        }
+                                        closer = t < bt;
                                 }
-                                closer = t64 < bt64;
+                                if (closer)
+                                {
+                                        best = f;
+                                        bt = t;
+                                        bt64 = t64;
+                                        b64 = is64;
+                                }
                         }
-                        else
-                        {
-                                closer = t < bt;
-                        }
-                        if (closer)
-                        {
-                                best = f;
-                                bt = t;
-                                bt64 = t64;
-                                b64 = is64;
-                        }
+                        __syncwarp();
                 }
-                __syncwarp();
         }
         *t_best = bt;
         return best;
 }
 
-// walk_step with the leaf's facets tested by leaf_closest_warp.  Every lane of the warp calls it
-// (active = false for lanes without a walk, whose result is ignored).
-template <int N, int RR = StageFit<N>::ROUNDS>
+// One step of the warp's walks: each lane locates the leaf at its probe and moves on to where its ray
+// leaves it, then the warp tests the leaves' facets; a hit counts when it lies inside the leaf.  The exit
+// needs no result of the tests, so its arithmetic runs while the records are on their way.  Every lane of
+// the warp calls it (active = false for lanes without a walk, whose result is ignored).
+template <int N, int RR>
 __device__ __forceinline__ int walk_step_warp(const MeshDev<N>& M, const float* bounds, Walk<N>& w, bool active, int retest,
                                               const float* raw_org, const float* raw_dir, float* t_out, int* facet_out,
                                               WalkStats* ws, int small_leaf = SMALL_LEAF)
 {
-        int status = W_MISS;
         bool leaf = false;
-        Leaf<N> lf;
-        int2 nd = make_int2(0, 0);
+        bool over = !active;
         if (active)
         {
-                status = W_RUNNING;
                 float probe[N];
                 w.probe(M.dist, probe);
                 if (++w.steps > 16384)
                 {
                         ws->error |= ERR_WALK_LIMIT;
-                        status = W_MISS;
+                        over = true;
                 }
-                else if (locate_leaf<N>(M, bounds, probe, w.pc, &lf, &nd, &ws->descent))
+                else if (locate_leaf<N>(M, bounds, probe, w.pc, &ws->descent))
                 {
                         ++ws->box_steps;
                         if (w.steps == 1)
@@ -1784,74 +1794,66 @@ __device__ __forceinline__ int walk_step_warp(const MeshDev<N>& M, const float* 
                                 // the origin is inside the tree: nothing travelled yet
                                 w.travelled = 0;
                         }
-                        if (w.travelled > w.tmax * 1.00001f + 1e-6f)
-                        {
-                                status = W_MISS;
-                        }
-                        else
-                        {
-                                leaf = true;
-                        }
+                        leaf = !(w.travelled > w.tmax * 1.00001f + 1e-6f);
+                        over = !leaf;
+                }
+                else if (w.steps != 1)
+                {
+                        over = true;
+                }
+                else
+                {
+                        // the origin is inside the root box but in no leaf (a gap between boxes): enter as
+                        // from outside
+                        walk_enter<N>(M, w);
                 }
         }
-        const int cnt = (leaf && nd.y > 0) ? nd.y : 0;
-        float t = FLT_MAX;
-        const int f = leaf_closest_warp<N, RR>(M, nd.x, cnt, w.ray, w.ao, w.raw, raw_org, raw_dir, retest, &t, ws,
-                                                small_leaf);
-        if (status != W_RUNNING)
-        {
-                return status;
-        }
+        WarpPool pool;
+        int pos[Stage<N, RR>::ROUNDS], own[Stage<N, RR>::ROUNDS];
+        pool_begin<N, RR>(M, w.pc.leaf.x, leaf ? w.pc.leaf.y : 0, small_leaf, &pool, pos, own);
         if (leaf)
         {
-                float sz[N];
-                level_size<N>(M, lf.level, sz);
-                if (f >= 0)
+                float org[N], size[N];
+                leaf_box<N>(M, bounds, w.pc, org, size);
+                const Exit<N> ex = leaf_exit<N>(org, size, w.cur, w.ray.dir);
+                over = !ex.ok;
+                if (ex.ok)
                 {
-                        float pt[N];
-                        ray_point<N>(w.ray, t, pt);
-                        bool inside = true;
 #pragma unroll
                         for (int i = 0; i < N; ++i)
                         {
-                                float d1 = lf.org[i] + sz[i];
-                                if (!(pt[i] <= d1) || !(-pt[i] <= -lf.org[i]))
-                                {
-                                        inside = false;
-                                }
+                                w.cur[i] = ex.ip[i];
                         }
-                        if (inside)
-                        {
-                                *t_out = t;
-                                *facet_out = f;
-                                return W_HIT;
-                        }
+                        // next probe: ip + dist * sg along the exit face's axis
+                        w.nudge = ex.nudge;
+                        w.travelled += ex.t;
                 }
-                const Exit<N> ex = leaf_exit<N>(lf.org, sz, w.cur, w.ray.dir);
-                if (!ex.ok)
-                {
-                        return W_MISS;
-                }
+        }
+        float t = FLT_MAX;
+        const int f = pool_closest<N, RR>(M, pool, pos, own, w.ray, w.ao, w.raw, raw_org, raw_dir, retest, &t, ws);
+        if (f >= 0)
+        {
+                float org[N], size[N], pt[N];
+                leaf_box<N>(M, bounds, w.pc, org, size);
+                ray_point<N>(w.ray, t, pt);
+                bool inside = true;
 #pragma unroll
                 for (int i = 0; i < N; ++i)
                 {
-                        w.cur[i] = ex.ip[i];
+                        float d1 = org[i] + size[i];
+                        if (!(pt[i] <= d1) || !(-pt[i] <= -org[i]))
+                        {
+                                inside = false;
+                        }
                 }
-                // next probe: ip + dist * sg along the exit face's axis
-                w.nudge = ex.nudge;
-                w.travelled += ex.t;
-        }
-        else
-        {
-                if (w.steps != 1)
+                if (inside)
                 {
-                        return W_MISS;
+                        *t_out = t;
+                        *facet_out = f;
+                        return W_HIT;
                 }
-                // the origin is inside the root box but in no leaf (a gap between boxes): enter as from
-                // outside
-                walk_enter<N>(M, w);
         }
-        return W_RUNNING;
+        return over ? W_MISS : W_RUNNING;
 }
 
 // What ray_intersection decides around the one mesh: the objects' approximate distances in stable

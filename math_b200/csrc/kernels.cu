@@ -100,6 +100,8 @@ __device__ __forceinline__ void flush_stats(unsigned long long* counters, const 
 // Fixed ray set: closest facet per ray through Mesh::intersect_approximate + intersect_precise
 // (the query of src/painter/shapes/test/test_mesh.cpp:139-152).
 
+constexpr int TRACE_ROUNDS = 1;  // staging rounds of the fixed-ray-set query's walk
+
 template <int N>
 __global__ void __launch_bounds__(BLOCK) k_trace_closest(__grid_constant__ const MeshDev<N> M, const float* __restrict__ org,
                                                          const float* __restrict__ dir, long long nrays, int retest,
@@ -142,7 +144,7 @@ __global__ void __launch_bounds__(BLOCK) k_trace_closest(__grid_constant__ const
         {
                 float t = 0;
                 int f = -1;
-                const int status = walk_step_warp<N>(M, bounds, w, walking, retest, org, dir, &t, &f, &ws);
+                const int status = walk_step_warp<N, TRACE_ROUNDS>(M, bounds, w, walking, retest, org, dir, &t, &f, &ws);
                 if (walking && status != W_RUNNING)
                 {
                         walking = false;
@@ -901,7 +903,8 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
                 {
                         float t = 0;
                         int f = -1;
-                        int status = walk_step_warp<N, R>(M, bounds, w, i >= 0, S.retest, nullptr, nullptr, &t, &f, &ws, S.walk_small);
+                        const int status = walk_step_warp<N, R>(M, bounds, w, i >= 0, S.retest, nullptr, nullptr, &t, &f, &ws,
+                                                                S.walk_small);
                         if (i >= 0 && status != W_RUNNING)
                         {
                                 float tt;
@@ -978,7 +981,8 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
                 {
                         float t = 0;
                         int f = -1;
-                        int status = walk_step_warp<N, R>(M, bounds, w, i >= 0, S.retest, nullptr, nullptr, &t, &f, &ws, S.walk_small);
+                        const int status = walk_step_warp<N, R>(M, bounds, w, i >= 0, S.retest, nullptr, nullptr, &t, &f, &ws,
+                                                                S.walk_small);
                         if (i >= 0 && status != W_RUNNING)
                         {
                                 if (!(status == W_HIT && t < dist))
@@ -1259,13 +1263,13 @@ void Wavefront<N>::carve(char* base, long long Q, int lights, bool smooth)
 }
 
 // The walk kernels' variant when the options leave it open: facet records read straight from global
-// memory (measured faster than staging them through shared memory on the configuration scenes, whose
-// leaves hold one or two facets per visit on average, so a warp's pooled list rarely fills a chunk).
+// memory (staged through shared memory in chunks of 32 they measured the same, n = 3, 4, 5 frames 2.49 /
+// 27.0 / 19.6 ms both ways: a step's pooled list holds about 20 tests, one round either way).
 template <int N>
 constexpr int DEFAULT_WALK_ROUNDS = -1;
 
 // Resident blocks of every kernel of an iteration, and the dynamic shared memory of the walk kernels
-// (they stage facet records there, leaf_closest_warp): computed once per dimension, on the first call,
+// (they stage facet records there, pool_stage): computed once per dimension, on the first call,
 // which the host makes before any capture (prepare_pass, nt_render_noalloc).
 template <int N>
 const LaunchSizes& Wavefront<N>::prepare()
@@ -1557,13 +1561,13 @@ cudaError_t launch_trace_closest(const MeshDev<N>& M, const float* org, const fl
                 return cudaSuccess;
         }
         static const bool smem_set =
-                cudaFuncSetAttribute(k_trace_closest<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Stage<N>::BYTES) ==
+                cudaFuncSetAttribute(k_trace_closest<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Stage<N, TRACE_ROUNDS>::BYTES) ==
                 cudaSuccess;
         if (!smem_set)
         {
                 return cudaErrorInvalidValue;
         }
-        k_trace_closest<N><<<(unsigned)grid_for<N>(nrays), BLOCK, Stage<N>::BYTES, st>>>(M, org, dir, nrays, retest, facet, t,
+        k_trace_closest<N><<<(unsigned)grid_for<N>(nrays), BLOCK, Stage<N, TRACE_ROUNDS>::BYTES, st>>>(M, org, dir, nrays, retest, facet, t,
                                                                                          counters);
         return cudaGetLastError();
 }
