@@ -185,7 +185,6 @@ struct PassDev
 enum Counter : int
 {
         C_ACTIVE_OUT = 0,
-        C_SHADOW = 1,
         C_ERROR = 2,
         C_RAYS = 3,
         C_FACET_TESTS = 4,
@@ -200,8 +199,6 @@ enum Counter : int
         C_SH_RETESTS = 12,
         // work cursors of the persistent extension and shadow kernels
         C_WORK_EXT = 13,
-        C_WORK_SH = 14,
-        C_SMOOTH = 15,     // entries of the smooth-normal shadow queue
         // wavefront control, kept on the device so that iterations need no host round trip
         C_Q_ACTIVE = 16,   // paths in the current queue
         C_Q_NEXT = 17,     // next fresh path of the pass (relative to PassDev::path_begin)
@@ -212,7 +209,12 @@ enum Counter : int
         // one-mesh scenes: extension rays that need the tree walk, compacted by k_plan_extend (the
         // shadow rays that need it are the shadow queue itself, C_SHADOW)
         C_WALK_EXT = 22,
-        C_COUNT = 23
+        // the shadow queues' lengths and the shadow kernels' work cursor, one for each parity of the
+        // iteration: an iteration's shadow walks may run beside the next one's first kernels
+        C_SHADOW = 23,
+        C_SMOOTH = 25,     // entries of the smooth-normal shadow queue
+        C_WORK_SH = 27,
+        C_COUNT = 29
 };
 
 enum ErrorBits : int

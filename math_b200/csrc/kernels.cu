@@ -350,7 +350,7 @@ __device__ __forceinline__ void accumulate(double* accum, uint32_t pixel, float 
 template <int N>
 __global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_constant__ const DevScene<N> S, const PassDev P, PathView<N> A, HitView<N> H,
                                                  PathView<N> B, ShadowView<N> SQ, ShadowView<N> SM, double* accum,
-                                                 unsigned long long* counters)
+                                                 unsigned long long* counters, int parity)
 {
         const long long count = (long long)counters[C_Q_ACTIVE];
         __shared__ int s_warp[BLOCK / 32];
@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_consta
                                 }
                                 shadow = walk;
                         }
-                        long long qo = compact_slot(shadow, counters + C_SHADOW, s_warp, &s_base);
+                        long long qo = compact_slot(shadow, counters + C_SHADOW + parity, s_warp, &s_base);
                         if (shadow)
                         {
 #pragma unroll
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_consta
                         if (S.smooth_normal)
                         {
                                 // block-uniform: every thread of the block takes part in the compaction
-                                long long bo = compact_slot(behind, counters + C_SMOOTH, s_warp, &s_base);
+                                long long bo = compact_slot(behind, counters + C_SMOOTH + parity, s_warp, &s_base);
                                 if (behind)
                                 {
 #pragma unroll
@@ -655,12 +655,12 @@ __global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_consta
 // shadow rays: light_source_is_visible (painter.cpp:172-186); visible -> add the light's share
 template <int N>
 __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>()) k_shadow(__grid_constant__ const DevScene<N> S, ShadowView<N> SQ, double* accum,
-                                                  unsigned long long* counters)
+                                                  unsigned long long* counters, int parity)
 {
-        const long long count = (long long)counters[C_SHADOW];
+        const long long count = (long long)counters[C_SHADOW + parity];
         WalkStats ws{0, 0, 0, 0, 0};
         long long rays = 0;
-        for (long long base = warp_take(counters + C_WORK_SH); base < count; base = warp_take(counters + C_WORK_SH))
+        for (long long base = warp_take(counters + C_WORK_SH + parity); base < count; base = warp_take(counters + C_WORK_SH + parity))
         {
                 long long i = base + (threadIdx.x & 31);
                 if (i < count)
@@ -690,11 +690,11 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>()) k_shadow(__grid_c
 // normals, only with smooth_normal), so one ray per thread through the general scene functions.
 template <int N>
 __global__ void __launch_bounds__(BLOCK) k_shadow_smooth(__grid_constant__ const DevScene<N> S, ShadowView<N> SM,
-                                                         double* accum, unsigned long long* counters)
+                                                         double* accum, unsigned long long* counters, int parity)
 {
         WalkStats ws{0, 0, 0, 0, 0};
         long long rays = 0;
-        const long long count = (long long)counters[C_SMOOTH];
+        const long long count = (long long)counters[C_SMOOTH + parity];
         for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
         {
                 Ray<N> r;
@@ -931,9 +931,10 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
 // at which each ray enters the mesh's root box): the walk runs up to the light's distance.
 template <int N, int R>
 __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
-        k_shadow_refill(__grid_constant__ const DevScene<N> S, ShadowView<N> SQ, double* accum, unsigned long long* counters)
+        k_shadow_refill(__grid_constant__ const DevScene<N> S, ShadowView<N> SQ, double* accum, unsigned long long* counters,
+                        int parity)
 {
-        const long long count = (long long)counters[C_SHADOW];
+        const long long count = (long long)counters[C_SHADOW + parity];
         const MeshDev<N>& M = S.mesh[0];
         const float* const bounds = walk_bounds<N>(M);
         WalkStats ws{0, 0, 0, 0, 0};
@@ -947,7 +948,7 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
         {
                 for (int round = 0; round < FILL_ROUNDS; ++round)
                 {
-                        const long long q = lane_refill(i < 0, counters + C_WORK_SH, count, &exhausted);
+                        const long long q = lane_refill(i < 0, counters + C_WORK_SH + parity, count, &exhausted);
                         if (q >= 0)
                         {
                                 const long long j = q;
@@ -1113,7 +1114,7 @@ __global__ void k_moments_reduce(long long npix, int spp, const double* __restri
 
 // Start of a wavefront iteration (one thread): refill the queue with fresh paths up to Q and clear the
 // per-iteration counters.
-__global__ void k_iter_begin(unsigned long long* c, long long total, long long Q)
+__global__ void k_iter_begin(unsigned long long* c, long long total, long long Q, int parity)
 {
         const long long active = (long long)c[C_Q_ACTIVE];
         const long long next = (long long)c[C_Q_NEXT];
@@ -1124,10 +1125,11 @@ __global__ void k_iter_begin(unsigned long long* c, long long total, long long Q
         c[C_Q_ACTIVE] = (unsigned long long)(active + fresh);
         c[C_Q_NEXT] = (unsigned long long)(next + fresh);
         c[C_WORK_EXT] = 0;
-        c[C_WORK_SH] = 0;
         c[C_ACTIVE_OUT] = 0;
-        c[C_SHADOW] = 0;
-        c[C_SMOOTH] = 0;
+        // this iteration's shadow queues (the previous iteration's may still be walked)
+        c[C_WORK_SH + parity] = 0;
+        c[C_SHADOW + parity] = 0;
+        c[C_SMOOTH + parity] = 0;
         c[C_WALK_EXT] = 0;
         if (active + fresh > 0)
         {
@@ -1295,7 +1297,7 @@ const LaunchSizes& Wavefront<N>::prepare()
 template <int N>
 void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, double* accum, unsigned long long* counters,
                                      long long total_paths, int parity, cudaStream_t st, KernelTimes* times,
-                                     cudaEvent_t* ev) const
+                                     cudaEvent_t* ev, const SideStream* side) const
 {
         const LaunchSizes& L = prepare();
         const long long extend_blocks = L.extend_blocks;
@@ -1322,7 +1324,7 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         HitView<N> H{hit_t, hit_obj, hit_facet};
         ShadowView<N> SQ{sq_f, sq_pix, Q * lights};
         ShadowView<N> SM{sm_f, sm_pix, Q * lights};
-        k_iter_begin<<<1, 1, 0, st>>>(counters, total_paths, Q);
+        k_iter_begin<<<1, 1, 0, st>>>(counters, total_paths, Q, parity);
         if (ev)
         {
                 cudaEventRecord(ev[0], st);
@@ -1368,7 +1370,12 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         {
                 cudaEventRecord(ev[3], st);
         }
-        k_shade<N><<<str_grid, BLOCK, 0, st>>>(S, P, A, H, B, SQ, SM, accum, counters);
+        if (side)
+        {
+                // the previous iteration's shadow walks read the queue that shading fills
+                cudaStreamWaitEvent(st, side->join, 0);
+        }
+        k_shade<N><<<str_grid, BLOCK, 0, st>>>(S, P, A, H, B, SQ, SM, accum, counters, parity);
         if (ev)
         {
                 cudaEventRecord(ev[4], st);
@@ -1377,32 +1384,43 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         {
                 cudaEventRecord(ev[5], st);
         }
+        cudaStream_t sh = st;
+        if (side)
+        {
+                sh = side->stream;
+                cudaEventRecord(side->fork, st);
+                cudaStreamWaitEvent(sh, side->fork, 0);
+        }
         if (one_mesh)
         {
                 if (vi == 0)
                 {
-                        k_shadow_refill<N, 0><<<sh_grid, BLOCK, 0, st>>>(S, SQ, accum, counters);
+                        k_shadow_refill<N, 0><<<sh_grid, BLOCK, 0, sh>>>(S, SQ, accum, counters, parity);
                 }
                 else if (vi == 1)
                 {
-                        k_shadow_refill<N, 1><<<sh_grid, BLOCK, Stage<N, 1>::BYTES, st>>>(S, SQ, accum, counters);
+                        k_shadow_refill<N, 1><<<sh_grid, BLOCK, Stage<N, 1>::BYTES, sh>>>(S, SQ, accum, counters, parity);
                 }
                 else if (vi == 2)
                 {
-                        k_shadow_refill<N, 2><<<sh_grid, BLOCK, Stage<N, 2>::BYTES, st>>>(S, SQ, accum, counters);
+                        k_shadow_refill<N, 2><<<sh_grid, BLOCK, Stage<N, 2>::BYTES, sh>>>(S, SQ, accum, counters, parity);
                 }
                 else
                 {
-                        k_shadow_refill<N, 4><<<sh_grid, BLOCK, Stage<N, 4>::BYTES, st>>>(S, SQ, accum, counters);
+                        k_shadow_refill<N, 4><<<sh_grid, BLOCK, Stage<N, 4>::BYTES, sh>>>(S, SQ, accum, counters, parity);
                 }
         }
         else
         {
-                k_shadow<N><<<sh_grid, BLOCK, 0, st>>>(S, SQ, accum, counters);
+                k_shadow<N><<<sh_grid, BLOCK, 0, sh>>>(S, SQ, accum, counters, parity);
         }
         if (smooth)
         {
-                k_shadow_smooth<N><<<str_grid, BLOCK, 0, st>>>(S, SM, accum, counters);
+                k_shadow_smooth<N><<<str_grid, BLOCK, 0, sh>>>(S, SM, accum, counters, parity);
+        }
+        if (side)
+        {
+                cudaEventRecord(side->join, sh);
         }
         if (ev)
         {
@@ -1417,54 +1435,52 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         }
 }
 
+// `count` iterations (an even number) in a row.  The shadow walks of one iteration and the ray
+// generation, plan and extension walk of the next do not depend on each other: with a side stream the
+// shadow walks go there, and the two persistent walk kernels fill each other's ends, when few long walks
+// are left, and the streaming kernels' gaps.
+template <int N>
+void Wavefront<N>::enqueue_iterations(const DevScene<N>& S, const PassDev& P, double* accum, unsigned long long* counters,
+                                      long long total_paths, int count, cudaStream_t st, KernelTimes* times,
+                                      const SideStream* side) const
+{
+        if (side)
+        {
+                cudaEventRecord(side->join, st);
+        }
+        for (int k = 0; k < count; ++k)
+        {
+                enqueue_iteration(S, P, accum, counters, total_paths, k & 1, st, times, nullptr, side);
+        }
+        if (side)
+        {
+                cudaStreamWaitEvent(st, side->join, 0);
+        }
+}
+
 template <int N>
 cudaError_t Wavefront<N>::run(const DevScene<N>& S, PassDev P, double* accum, unsigned long long* counters,
                               unsigned long long* host_counters, long long total_paths, cudaStream_t st, KernelTimes* times,
-                              bool timing, const volatile int* stop, bool use_graph, int batch)
+                              bool timing, const volatile int* stop, int batch, const SideStream* side)
 {
         const bool smooth = S.smooth_normal != 0;
         if (smooth && !sm_f)
         {
                 return cudaErrorInvalidValue;  // the pool was carved without the smooth-normal queue
         }
-        prepare();  // kernel attributes and occupancy, outside the capture below
-        // iterations between host checks of the done flag (a pass takes tens of iterations; the few
-        // that run after it is done find empty queues and return at once)
-        const int BATCH = std::max(1, batch);
+        prepare();  // kernel attributes and occupancy
+        // iterations between host checks of the done flag (the few that run after the pass is done find
+        // empty queues and return at once); an even number, so that the queue parity is the same at the
+        // start of every batch.  They are launched directly: the launches of a batch take less time than its
+        // kernels, and capturing and instantiating a graph per pass took longer than replaying it saved
+        // (one pass of 36,864 paths 0.72 ms as a graph, 0.63 direct, 0.48 with the side stream; n = 3 frame
+        // of 2.56 M paths 2.39 / 2.27 / 1.90; n = 4 of 56.6 M 24.7 / 24.5 / 23.9; n = 5 of 30.1 M 17.8 / 17.8 /
+        // 16.3)
+        const int even = std::max(1, batch) + (std::max(1, batch) & 1);
         cudaError_t e = cudaMemsetAsync(counters + C_Q_ACTIVE, 0, (C_COUNT - C_Q_ACTIVE) * sizeof(unsigned long long), st);
         if (e != cudaSuccess)
         {
                 return e;
-        }
-        cudaGraphExec_t exec = nullptr;
-        if (use_graph && !timing)
-        {
-                // the BATCH iterations are captured once per pass and replayed as one graph launch
-                // (BATCH even, so that the queue parity is the same at the start of every replay)
-                const int even = BATCH + (BATCH & 1);
-                cudaGraph_t graph = nullptr;
-                e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-                if (e == cudaSuccess)
-                {
-                        for (int k = 0; k < even; ++k)
-                        {
-                                enqueue_iteration(S, P, accum, counters, total_paths, k & 1, st, nullptr, nullptr);
-                        }
-                        e = cudaStreamEndCapture(st, &graph);
-                        if (e == cudaSuccess)
-                        {
-                                e = cudaGraphInstantiate(&exec, graph, 0);
-                                cudaGraphDestroy(graph);
-                        }
-                }
-                if (e != cudaSuccess)
-                {
-                        // capture unavailable (e.g. the caller's stream is itself being captured):
-                        // enqueue the iterations directly
-                        cudaGetLastError();
-                        exec = nullptr;
-                        e = cudaSuccess;
-                }
         }
         cudaEvent_t ev[8];
         if (timing)
@@ -1474,8 +1490,6 @@ cudaError_t Wavefront<N>::run(const DevScene<N>& S, PassDev P, double* accum, un
                         cudaEventCreate(&v);
                 }
         }
-        const int per_replay = BATCH + (BATCH & 1);
-        int parity = 0;
         while (true)
         {
                 if (stop && *stop)
@@ -1484,10 +1498,9 @@ cudaError_t Wavefront<N>::run(const DevScene<N>& S, PassDev P, double* accum, un
                 }
                 if (timing)
                 {
-                        for (int k = 0; k < BATCH; ++k)
+                        for (int k = 0; k < even; ++k)
                         {
-                                enqueue_iteration(S, P, accum, counters, total_paths, parity, st, times, ev);
-                                parity ^= 1;
+                                enqueue_iteration(S, P, accum, counters, total_paths, k & 1, st, times, ev, nullptr);
                                 cudaEventRecord(ev[7], st);
                                 cudaEventSynchronize(ev[7]);
                                 float ms;
@@ -1505,24 +1518,9 @@ cudaError_t Wavefront<N>::run(const DevScene<N>& S, PassDev P, double* accum, un
                                 times->shadow_ms += ms;
                         }
                 }
-                else if (exec)
-                {
-                        e = cudaGraphLaunch(exec, st);
-                        if (e != cudaSuccess)
-                        {
-                                break;
-                        }
-                        times->launches += (long long)per_replay * iteration_launches(smooth, S.nmesh == 1);
-                        times->extend_launches += per_replay;
-                        times->shadow_launches += per_replay;
-                }
                 else
                 {
-                        for (int k = 0; k < BATCH; ++k)
-                        {
-                                enqueue_iteration(S, P, accum, counters, total_paths, parity, st, times, nullptr);
-                                parity ^= 1;
-                        }
+                        enqueue_iterations(S, P, accum, counters, total_paths, even, st, times, side);
                 }
                 e = cudaMemcpyAsync(host_counters, counters, C_COUNT * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
                 if (e == cudaSuccess)
@@ -1533,10 +1531,6 @@ cudaError_t Wavefront<N>::run(const DevScene<N>& S, PassDev P, double* accum, un
                 {
                         break;
                 }
-        }
-        if (exec)
-        {
-                cudaGraphExecDestroy(exec);
         }
         if (timing)
         {

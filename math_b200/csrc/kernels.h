@@ -36,6 +36,15 @@ struct LaunchSizes
         long long stream_blocks = 1;
 };
 
+// A second stream for the kernels of an iteration that the next one does not wait for, and the events that
+// tie it to the pass's stream.
+struct SideStream
+{
+        cudaStream_t stream = nullptr;
+        cudaEvent_t fork = nullptr;
+        cudaEvent_t join = nullptr;
+};
+
 // Wavefront path pool: path state A/B (double-buffered, compacted every bounce), the hit record and
 // the shadow-ray queue, all carved out of one caller-provided device allocation.
 template <int N>
@@ -73,18 +82,22 @@ struct Wavefront
         // pinned host mirror of all of them.
         // times: launch counts always, per-kernel device times when timing (events around every
         // launch); stop: optional host flag polled once per wavefront iteration (between launches).
-        // The iterations run in batches of `batch` captured as one CUDA graph (use_graph; else enqueued
-        // directly), the host reading the done flag after each batch.
+        // The iterations run in batches of `batch`, the host reading the done flag after each batch; side:
+        // the stream of the shadow walks (enqueue_iterations; null: one stream for everything).
         cudaError_t run(const DevScene<N>& S, PassDev P, double* accum, unsigned long long* counters,
                         unsigned long long* host_counters, long long total_paths, cudaStream_t st, KernelTimes* times,
-                        bool timing, const volatile int* stop, bool use_graph = true, int batch = 4);
+                        bool timing, const volatile int* stop, int batch = 4, const SideStream* side = nullptr);
 
         // One wavefront iteration on stream st (k_iter_begin .. k_iter_end; the queue sizes live in
         // counters, so nothing waits for the host).  parity selects which double-buffered queue is
-        // current; ev (8 events, optional) are recorded around the kernel kinds.  Capturable.
+        // current; ev (8 events, optional) are recorded around the kernel kinds; side (optional): the shadow
+        // walks' stream, joined by the next iteration's shading.  Capturable.
         void enqueue_iteration(const DevScene<N>& S, const PassDev& P, double* accum, unsigned long long* counters,
                                long long total_paths, int parity, cudaStream_t st, KernelTimes* times,
-                               cudaEvent_t* ev) const;
+                               cudaEvent_t* ev, const SideStream* side) const;
+        void enqueue_iterations(const DevScene<N>& S, const PassDev& P, double* accum, unsigned long long* counters,
+                                long long total_paths, int count, cudaStream_t st, KernelTimes* times,
+                                const SideStream* side) const;
         static int iteration_launches(bool smooth, bool one_mesh)
         {
                 return 6 + (smooth ? 1 : 0) + (one_mesh ? 1 : 0);

@@ -331,6 +331,7 @@ struct nt_scene
         float ray_offset = 0;
         // device
         cudaStream_t stream = nullptr;
+        ntrace::SideStream side;  // the shadow walks' stream (Wavefront::enqueue_iterations)
         DevBuf accum;
         DevBuf pool;
         long long pool_paths = 0;
@@ -369,6 +370,17 @@ struct nt_scene
                 if (host_counters)
                 {
                         cudaFreeHost(host_counters);
+                }
+                if (side.stream)
+                {
+                        cudaStreamDestroy(side.stream);
+                }
+                for (cudaEvent_t e : {side.fork, side.join})
+                {
+                        if (e)
+                        {
+                                cudaEventDestroy(e);
+                        }
                 }
                 if (stream)
                 {
@@ -1060,6 +1072,12 @@ void build_scene(nt_scene* s, unsigned threads, bool host_only, bool tree_on_gpu
         {
                 check_cuda(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "cudaStreamCreate");
         }
+        if (!host_only && !s->side.join)
+        {
+                check_cuda(cudaStreamCreateWithFlags(&s->side.stream, cudaStreamNonBlocking), "cudaStreamCreate");
+                check_cuda(cudaEventCreateWithFlags(&s->side.fork, cudaEventDisableTiming), "cudaEventCreate");
+                check_cuda(cudaEventCreateWithFlags(&s->side.join, cudaEventDisableTiming), "cudaEventCreate");
+        }
         for (auto& m : s->meshes)
         {
                 if (!m.ready)
@@ -1372,8 +1390,8 @@ struct PassJob
         KernelTimes times;
         std::chrono::steady_clock::time_point t0;
         virtual ~PassJob() = default;
-        // one wavefront iteration of this pass on stream st
-        virtual void enqueue(int parity, cudaStream_t st) = 0;
+        // `count` wavefront iterations of this pass on stream st
+        virtual void enqueue(int count, cudaStream_t st) = 0;
         // the whole pass on the scene's stream
         virtual cudaError_t run(const nt_render_opts& o) = 0;
 };
@@ -1385,14 +1403,14 @@ struct PassJobN final : PassJob
         PassDev P{};
         Wavefront<N> W;
         double* accum = nullptr;
-        void enqueue(int parity, cudaStream_t st) override
+        void enqueue(int count, cudaStream_t st) override
         {
-                W.enqueue_iteration(S, P, accum, s->counters.as<unsigned long long>(), total, parity, st, nullptr, nullptr);
+                W.enqueue_iterations(S, P, accum, s->counters.as<unsigned long long>(), total, count, st, nullptr, &s->side);
         }
         cudaError_t run(const nt_render_opts& o) override
         {
                 return W.run(S, P, accum, s->counters.as<unsigned long long>(), s->host_counters, total, s->stream, &times,
-                             o.timing != 0, o.stop, true, o.graph_iterations > 0 ? o.graph_iterations : 4);
+                             o.timing != 0, o.stop, o.graph_iterations > 0 ? o.graph_iterations : 4, &s->side);
         }
 };
 
@@ -1655,8 +1673,7 @@ void render_noalloc(nt_scene* s, const nt_render_opts& o, double* d_accum, long 
         check_cuda(cudaMemsetAsync(counters, 0, C_COUNT * sizeof(unsigned long long), st), "memset counters");
         unsigned long long host_counters[C_COUNT] = {};
         KernelTimes times;
-        // the iterations are enqueued directly, not through a CUDA graph: instantiating a graph may allocate
-        check_cuda(W.run(S, P, d_accum, counters, host_counters, total, st, &times, false, o.stop, false), "render");
+        check_cuda(W.run(S, P, d_accum, counters, host_counters, total, st, &times, false, o.stop), "render");
         check_cuda(cudaMemcpyAsync(host_counters, counters, C_COUNT * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st),
                    "counters");
         check_cuda(cudaStreamSynchronize(st), "render sync");
@@ -2553,12 +2570,9 @@ int nt_render_batch(nt_scene* const* scenes, int count, const nt_render_opts* op
                 {
                         nt_scene* s = scenes[i];
                         e = cudaStreamWaitEvent(s->stream, events[count], 0);
-                        for (int k = 0; k < per && e == cudaSuccess; ++k)
-                        {
-                                jobs[i]->enqueue(k & 1, s->stream);
-                        }
                         if (e == cudaSuccess)
                         {
+                                jobs[i]->enqueue(per, s->stream);
                                 e = cudaMemcpyAsync(s->host_counters, s->counters.p, C_COUNT * sizeof(unsigned long long),
                                                     cudaMemcpyDeviceToHost, s->stream);
                         }
