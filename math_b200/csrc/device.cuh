@@ -2020,22 +2020,6 @@ __device__ __forceinline__ bool smooth_normal(const MeshDev<N>& M, int facet, co
 // ------------------------------------------------------------------------------------------------
 // Sampling (sphere.h:87-116, complement.h:71-200)
 
-template <int N>
-__device__ __forceinline__ void ortho_nn_dev(const float (*v)[N], float* r);
-
-template <>
-__device__ __forceinline__ void ortho_nn_dev<4>(const float (*v)[4], float* r)
-{
-        r[0] = +v[0][1] * (v[1][2] * v[2][3] - v[1][3] * v[2][2]) - v[0][2] * (v[1][1] * v[2][3] - v[1][3] * v[2][1]) +
-               v[0][3] * (v[1][1] * v[2][2] - v[1][2] * v[2][1]);
-        r[1] = -v[0][0] * (v[1][2] * v[2][3] - v[1][3] * v[2][2]) + v[0][2] * (v[1][0] * v[2][3] - v[1][3] * v[2][0]) -
-               v[0][3] * (v[1][0] * v[2][2] - v[1][2] * v[2][0]);
-        r[2] = +v[0][0] * (v[1][1] * v[2][3] - v[1][3] * v[2][1]) - v[0][1] * (v[1][0] * v[2][3] - v[1][3] * v[2][0]) +
-               v[0][3] * (v[1][0] * v[2][1] - v[1][1] * v[2][0]);
-        r[3] = -v[0][0] * (v[1][1] * v[2][2] - v[1][2] * v[2][1]) + v[0][1] * (v[1][0] * v[2][2] - v[1][2] * v[2][0]) -
-               v[0][2] * (v[1][0] * v[2][1] - v[1][1] * v[2][0]);
-}
-
 __device__ __forceinline__ void cross3(const float* a, const float* b, float* r)
 {
         r[0] = +(a[1] * b[2] - a[2] * b[1]);
@@ -2061,64 +2045,6 @@ __device__ __forceinline__ void complement(const float* u, float (*basis)[N])
                 cross3(u, nc, basis[0]);
                 vnormalize<3>(basis[0]);
                 cross3(u, basis[0], basis[1]);
-        }
-        else if constexpr (N == 4)
-        {
-                int exclude_axis = 0;
-                for (; exclude_axis < N - 2; ++exclude_axis)
-                {
-                        if (fabsf(u[exclude_axis]) > LIMIT)
-                        {
-                                break;
-                        }
-                }
-                float sb[N - 1][N];
-#pragma unroll
-                for (int k = 0; k < N; ++k)
-                {
-                        sb[N - 2][k] = u[k];
-                }
-                int num = 0;
-                for (int i = 0; num < N - 2; ++i)
-                {
-                        if (i != exclude_axis)
-                        {
-#pragma unroll
-                                for (int k = 0; k < N; ++k)
-                                {
-                                        sb[num][k] = (k == i) ? 1.0f : 0.0f;
-                                }
-                                ++num;
-                        }
-                }
-#pragma unroll
-                for (int i = 0; i < N - 2; ++i)
-                {
-                        float o[N];
-                        ortho_nn_dev<N>(sb, o);
-                        vnormalize<N>(o);
-#pragma unroll
-                        for (int k = 0; k < N; ++k)
-                        {
-                                sb[i][k] = o[k];
-                        }
-                }
-                float o[N];
-                ortho_nn_dev<N>(sb, o);
-#pragma unroll
-                for (int k = 0; k < N; ++k)
-                {
-                        sb[N - 2][k] = o[k];
-                }
-#pragma unroll
-                for (int i = 0; i < N - 1; ++i)
-                {
-#pragma unroll
-                        for (int k = 0; k < N; ++k)
-                        {
-                                basis[i][k] = sb[i][k];
-                        }
-                }
         }
         else
         {
@@ -2201,53 +2127,177 @@ __device__ __forceinline__ float radial_scale(float len2)
         }
 }
 
-// random_cosine_weighted_on_hemisphere with the ball point by rejection; false if the attempt
-// bound ran out (probability < 1e-19 per call)
+// One attempt at a point of the unit ball in N - 1 dimensions, by rejection (sphere.h:42-56): attempt
+// `attempt` of the path's stream.
 template <int N>
-__device__ bool cosine_hemisphere(uint32_t k0, uint32_t k1, unsigned long long path, uint32_t stream, const float* normal,
-                                  float* res)
+__device__ __forceinline__ bool ball_attempt(uint32_t k0, uint32_t k1, unsigned long long path, uint32_t stream,
+                                             uint32_t attempt, float* v, float* len2)
 {
         constexpr int M = N - 1;
-        float v[M];
-        float len2 = 0;
-        bool ok = false;
-        for (uint32_t attempt = 0; attempt < 256; ++attempt)
+        float u[8];
+        if constexpr (M <= 4)
         {
-                float u[8];
-                if constexpr (M <= 4)
+                float4 a = rng4(k0, k1, path, stream, attempt);
+                u[0] = a.x;
+                u[1] = a.y;
+                u[2] = a.z;
+                u[3] = a.w;
+        }
+        else
+        {
+                float4 a = rng4(k0, k1, path, stream, 2 * attempt);
+                float4 b = rng4(k0, k1, path, stream, 2 * attempt + 1);
+                u[0] = a.x;
+                u[1] = a.y;
+                u[2] = a.z;
+                u[3] = a.w;
+                u[4] = b.x;
+        }
+#pragma unroll
+        for (int j = 0; j < M; ++j)
+        {
+                v[j] = 2.0f * u[j] - 1.0f;
+        }
+        *len2 = vdot<M>(v, v);
+        return *len2 <= 1 && *len2 > 0;
+}
+
+constexpr uint32_t BALL_ATTEMPTS = 256;
+
+// A ball point by rejection; false: the bound of attempts ran out (probability < 1e-19).
+template <int N>
+__device__ __forceinline__ bool ball_point(uint32_t k0, uint32_t k1, unsigned long long path, uint32_t stream, float* v,
+                                           float* len2)
+{
+        for (uint32_t attempt = 0; attempt < BALL_ATTEMPTS; ++attempt)
+        {
+                if (ball_attempt<N>(k0, k1, path, stream, attempt, v, len2))
                 {
-                        float4 a = rng4(k0, k1, path, stream, attempt);
-                        u[0] = a.x;
-                        u[1] = a.y;
-                        u[2] = a.z;
-                        u[3] = a.w;
+                        return true;
                 }
-                else
+        }
+        return false;
+}
+
+// The ball point of every lane that needs one, n >= 5: there an attempt succeeds with probability 0.31 or
+// 0.16 and a per-lane loop runs as long as the unluckiest of 32 lanes, 10 to 20 attempts; here the
+// warp's lanes are dealt out over the lanes still open, each trying one of its owner's next attempts
+// (the random numbers are addressed by attempt, so their order does not matter), and the owner takes the
+// earliest accepted one.  At n = 3 and 4 (0.79, 0.52) the dealing costs what it saves.  Every lane of
+// the warp calls it.
+template <int N>
+__device__ __forceinline__ bool ball_point_warp(bool need, uint32_t k0, uint32_t k1, unsigned long long path,
+                                                uint32_t stream, float* v, float* len2)
+{
+        constexpr int M = N - 1;
+        constexpr uint32_t ATTEMPTS = BALL_ATTEMPTS;
+        const unsigned full = 0xffffffffu;
+        const int lane = threadIdx.x & 31;
+        __shared__ int s_owner[WALK_BLOCK];
+        int* const owner = s_owner + (threadIdx.x & ~31);
+        bool done = !need;
+        uint32_t next = 0;
+        while (true)
+        {
+                const unsigned open = __ballot_sync(full, !done && next < ATTEMPTS);
+                if (!open)
                 {
-                        float4 a = rng4(k0, k1, path, stream, 2 * attempt);
-                        float4 b = rng4(k0, k1, path, stream, 2 * attempt + 1);
-                        u[0] = a.x;
-                        u[1] = a.y;
-                        u[2] = a.z;
-                        u[3] = a.w;
-                        u[4] = b.x;
+                        break;
                 }
+                const int count = __popc(open);
+                const bool mine_open = (open >> lane) & 1u;
+                const int rank = __popc(open & ((1u << lane) - 1));
+                if (mine_open)
+                {
+                        owner[rank] = lane;
+                }
+                __syncwarp();
+                // lane L tries attempt L / count (counted from the owner's next) of the open lane of rank L % count
+                const int offset = (int)(((float)lane + 0.5f) * __frcp_rn((float)count));
+                const int from = owner[lane - offset * count];
+                const unsigned long long o_path = __shfl_sync(full, path, from);
+                const uint32_t o_stream = __shfl_sync(full, stream, from);
+                const uint32_t attempt = __shfl_sync(full, next, from) + offset;
+                float tv[M], tl = 0;
+                const bool hit = attempt < ATTEMPTS && ball_attempt<N>(k0, k1, o_path, o_stream, attempt, tv, &tl);
+                const unsigned hits = __ballot_sync(full, hit);
+                // the lanes of rank `rank`: rank, rank + count, ...
+                unsigned pattern = 1;
+                for (int s = count; s < 32; s <<= 1)
+                {
+                        pattern |= pattern << s;
+                }
+                const unsigned mine = mine_open ? hits & (pattern << rank) : 0u;
+                const int src = mine ? __ffs(mine) - 1 : lane;
 #pragma unroll
                 for (int j = 0; j < M; ++j)
                 {
-                        v[j] = 2.0f * u[j] - 1.0f;
+                        const float x = __shfl_sync(full, tv[j], src);
+                        v[j] = mine ? x : v[j];
                 }
-                len2 = vdot<M>(v, v);
-                if (len2 <= 1 && len2 > 0)
-                {
-                        ok = true;
-                        break;
-                }
+                const float x = __shfl_sync(full, tl, src);
+                *len2 = mine ? x : *len2;
+                done = done || mine != 0;
+                next += __popc(pattern << rank);
+                __syncwarp();
         }
-        if (!ok)
-        {
-                return false;
-        }
+        return done;
+}
+
+// nz * u + sum_j v_j * basis_j with the orthogonal complement of u at n = 4 (complement.h:71-200: the
+// generalised cross products o1 = (e_a, e_b, u), o2 = (o1, e_b, u), both normalised, and o3 = (o1, o2, u),
+// e_a and e_b the unit axes left after the excluded one).  The rows e_a and e_b leave two, three and four
+// components of the products, each a product or a difference of two: written out in the frame w that
+// has the excluded axis first, then e_a, e_b and the last axis, every operation that is left is one of the
+// full determinants', in their order (a permutation of the axes changes signs only).  64 registers hold
+// what the three full determinants spilled.
+__device__ __forceinline__ void hemisphere_vector4(const float* u, float nz, const float* v, float* res)
+{
+        const float LIMIT = 0.1f;
+        const bool ex0 = fabsf(u[0]) > LIMIT;
+        const bool ex1 = !ex0 && fabsf(u[1]) > LIMIT;
+        const float w0 = ex0 ? u[0] : (ex1 ? u[1] : u[2]);
+        const float w1 = ex0 ? u[1] : u[0];
+        const float w2 = ex0 || ex1 ? u[2] : u[1];
+        const float w3 = u[3];
+        // o1 = (w3, 0, 0, -w0), with the sign of the permutation (odd when axis 1 is excluded)
+        float p = ex1 ? -w3 : w3;
+        float q = ex1 ? w0 : -w0;
+        const float l1 = __fsqrt_rn(__fmaf_rn(q, q, p * p));
+        p = __fdiv_rn(p, l1);
+        q = __fdiv_rn(q, l1);
+        // o2 = (-(q w1), q w0 - p w3, 0, p w1) of the unsigned o1
+        const float ps = ex1 ? -p : p;
+        const float qs = ex1 ? -q : q;
+        float a = -(qs * w1);
+        float b = qs * w0 - ps * w3;
+        float c = ps * w1;
+        // the squares in the order of the axes: axis 0 is w0's, or w1's when another one is excluded
+        const float x = ex0 ? a : b;
+        const float y = ex0 ? b : a;
+        const float l2 = __fsqrt_rn(__fmaf_rn(c, c, __fmaf_rn(y, y, x * x)));
+        a = __fdiv_rn(a, l2);
+        b = __fdiv_rn(b, l2);
+        c = __fdiv_rn(c, l2);
+        const float d0 = qs * (b * w2);
+        const float d1 = ps * (c * w2) - qs * (a * w2);
+        const float d2 = ps * (b * w3 - c * w1) + qs * (a * w1 - b * w0);
+        const float d3 = -(ps * (b * w2));
+        const float r0 = nz * w0 + v[0] * p + v[1] * a + v[2] * d0;
+        const float r1 = nz * w1 + v[1] * b + v[2] * d1;
+        const float r2 = nz * w2 + v[2] * d2;
+        const float r3 = nz * w3 + v[0] * q + v[1] * c + v[2] * d3;
+        res[0] = ex0 ? r0 : r1;
+        res[1] = ex0 ? r1 : (ex1 ? r0 : r2);
+        res[2] = ex0 || ex1 ? r2 : r0;
+        res[3] = r3;
+}
+
+// random_cosine_weighted_on_hemisphere (sphere.h:87-116) from the ball point v, len2
+template <int N>
+__device__ __forceinline__ void cosine_hemisphere(float* v, float len2, const float* normal, float* res)
+{
+        constexpr int M = N - 1;
         if constexpr (N >= 4)
         {
                 float k = radial_scale<N>(len2);
@@ -2259,23 +2309,30 @@ __device__ bool cosine_hemisphere(uint32_t k0, uint32_t k1, unsigned long long p
                 len2 *= k * k;
         }
         float nz = __fsqrt_rn(1.0f - len2);
-        float basis[N - 1][N];
-        complement<N>(normal, basis);
-#pragma unroll
-        for (int k = 0; k < N; ++k)
+        if constexpr (N == 4)
         {
-                res[k] = nz * normal[k];
+                hemisphere_vector4(normal, nz, v, res);
+                return;
         }
-#pragma unroll
-        for (int j = 0; j < M; ++j)
+        else
         {
+                float basis[N - 1][N];
+                complement<N>(normal, basis);
 #pragma unroll
                 for (int k = 0; k < N; ++k)
                 {
-                        res[k] = res[k] + v[j] * basis[j][k];
+                        res[k] = nz * normal[k];
+                }
+#pragma unroll
+                for (int j = 0; j < M; ++j)
+                {
+#pragma unroll
+                        for (int k = 0; k < N; ++k)
+                        {
+                                res[k] = res[k] + v[j] * basis[j][k];
+                        }
                 }
         }
-        return true;
 }
 
 // Projector::ray (projector.h:102-275)

@@ -162,6 +162,14 @@ struct DevScene
                              // are tested per lane instead of pooled across the warp
 };
 
+// Division of a 31-bit number by a constant: n / d = (n m) >> s with m = floor(2^s / d) + 1 and s = 31 +
+// ceil(log2 d), which is exact for n < 2^31 (Granlund and Montgomery, "Division by invariant integers
+// using multiplication", 1994).
+struct FastDiv
+{
+        uint32_t d, m, s;
+};
+
 // Render-pass constants.
 struct PassDev
 {
@@ -179,6 +187,9 @@ struct PassDev
         const long long* list;    // non-null: the pass paints these pixels (linear indices) only; path g
                                   // is sample g % spp_eff of list entry g / spp_eff, and the queues carry
                                   // the entry (the accumulator has one slot per entry)
+        int small;                // 1: path and pixel numbers are below 2^31 and divided by the constants below
+        FastDiv by_spp, by_k;     // spp_eff, k1d
+        FastDiv by_screen[5];     // the screen sizes
 };
 
 // Device-wide counters (one int64 each).

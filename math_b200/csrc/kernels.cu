@@ -1,6 +1,6 @@
 // sm_100a kernels of the n-space path tracer: the fixed-ray-set closest-hit query and the
 // wavefront (ray generation, extension, shading, shadow rays, accumulation) with path and shadow
-// queues compacted by warp ballot plus block prefix sums.
+// queues compacted by warp ballots.
 #include "device.cuh"
 #include "kernels.h"
 
@@ -18,27 +18,21 @@ constexpr int BLOCK = WALK_BLOCK;  // every wavefront kernel's block size
 #define NT_WALK_MIN_BLOCKS 5
 #endif
 constexpr int WALK_MIN_BLOCKS = NT_WALK_MIN_BLOCKS;
-// resident blocks per SM asked of the shading kernel (a build-time option): 8 blocks of 128 caps it at
-// 64 registers, 32 warps per SM instead of 16 at the 108 it takes uncapped; the kernel is bound by
-// latency at that occupancy (ncu: 47 % issue, 13 % of DRAM bandwidth), and the n = 4 frame measured
-// 40.5 -> 38.3 ms with the cap despite a few spilled registers
-#ifndef NT_SHADE_MIN_BLOCKS
-#define NT_SHADE_MIN_BLOCKS 8
-#endif
-constexpr int SHADE_MIN_BLOCKS = NT_SHADE_MIN_BLOCKS;
+// resident blocks per SM asked of the shading kernel: it is bound by its instructions and their latency
+// (ncu, n = 4: issue slots 63 % busy, 16 % of DRAM throughput).  At n = 3 8 blocks of 128 fit 64 registers
+// without spills; above that 6 (80 registers) spill less (n = 4 frame: shading 7.29 ms with 8, 6.96 with
+// 6; n = 5 6.44 and 6.22; n = 3 0.376 and 0.400)
+template <int N>
+constexpr int shade_min_blocks()
+{
+        return N == 3 ? 8 : 6;
+}
 // at n = 6 the walk state is larger: one block fewer, so that 128 registers fit without spills
 template <int N>
 constexpr int walk_min_blocks()
 {
         return (N >= 6 && WALK_MIN_BLOCKS > 1) ? WALK_MIN_BLOCKS - 1 : WALK_MIN_BLOCKS;
 }
-// fill rounds per iteration of the lane-refill walks (1 measured faster than 2, 4, 8 or 16: a lane
-// whose new ray needs no walk waits for the next iteration rather than holding up the warp)
-#ifndef NT_FILL_ROUNDS
-#define NT_FILL_ROUNDS 1
-#endif
-constexpr int FILL_ROUNDS = NT_FILL_ROUNDS;
-
 __device__ __forceinline__ unsigned lanemask_lt()
 {
         unsigned m;
@@ -46,34 +40,78 @@ __device__ __forceinline__ unsigned lanemask_lt()
         return m;
 }
 
-// Block-wide stream compaction slot: every thread of the block must call it (flag may be false).
-// Warp ballot + popc give the in-warp prefix, a shared-memory scan over warps gives the block
-// offset, and one atomic per block reserves the block's range in the output queue.
-__device__ __forceinline__ long long compact_slot(bool flag, unsigned long long* counter, int* s_warp, long long* s_base)
+// Stream compaction slot of a warp: every lane calls it (flag may be false).  Warp ballot + popc give the
+// prefix, one atomic per warp reserves the warp's range in the output queue.
+__device__ __forceinline__ long long compact_slot(bool flag, unsigned long long* counter)
 {
-        const int lane = threadIdx.x & 31;
-        const int warp = threadIdx.x >> 5;
-        unsigned ballot = __ballot_sync(0xffffffffu, flag);
-        if (lane == 0)
+        const unsigned ballot = __ballot_sync(0xffffffffu, flag);
+        if (!ballot)
         {
-                s_warp[warp] = __popc(ballot);
+                return -1;
+        }
+        const int leader = __ffs(ballot) - 1;
+        unsigned long long base = 0;
+        if ((int)(threadIdx.x & 31) == leader)
+        {
+                base = atomicAdd(counter, (unsigned long long)__popc(ballot));
+        }
+        base = __shfl_sync(0xffffffffu, base, leader);
+        return flag ? (long long)base + __popc(ballot & lanemask_lt()) : -1;
+}
+
+// The same for a block: every thread calls it; one atomic per block, and two barriers.  Consecutive calls
+// alternate between the two halves of CompactShared (turn).
+struct CompactShared
+{
+        int warp[2][BLOCK / 32];
+        long long base[2];
+};
+
+__device__ __forceinline__ long long compact_slot_block(bool flag, unsigned long long* counter, CompactShared* sh, int* turn)
+{
+        const int warp = threadIdx.x >> 5;
+        const int b = *turn;
+        *turn ^= 1;
+        const unsigned ballot = __ballot_sync(0xffffffffu, flag);
+        if ((threadIdx.x & 31) == 0)
+        {
+                sh->warp[b][warp] = __popc(ballot);
         }
         __syncthreads();
+        int before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < BLOCK / 32; ++w)
+        {
+                const int c = sh->warp[b][w];
+                before += w < warp ? c : 0;
+                total += c;
+        }
+        if (total == 0)
+        {
+                return -1;
+        }
         if (threadIdx.x == 0)
         {
-                int total = 0;
-                for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
-                {
-                        int c = s_warp[w];
-                        s_warp[w] = total;
-                        total += c;
-                }
-                *s_base = total ? (long long)atomicAdd(counter, (unsigned long long)total) : 0;
+                sh->base[b] = (long long)atomicAdd(counter, (unsigned long long)total);
         }
         __syncthreads();
-        long long slot = *s_base + s_warp[warp] + __popc(ballot & lanemask_lt());
-        __syncthreads();
-        return flag ? slot : -1;
+        return flag ? sh->base[b] + before + __popc(ballot & lanemask_lt()) : -1;
+}
+
+// The shading kernel's choice.  Its three queues take two atomics per warp and tile; at n >= 4 a tile's
+// arithmetic covers them and the barriers cost more (n = 4 frame: shading 8.3 ms by block, 7.4 by warp),
+// at n = 3 the rate of atomics on one address bounds it (0.36 ms by block, 0.44 by warp).
+template <int N>
+__device__ __forceinline__ long long shade_slot(bool flag, unsigned long long* counter, CompactShared* sh, int* turn)
+{
+        if constexpr (N == 3)
+        {
+                return compact_slot_block(flag, counter, sh, turn);
+        }
+        else
+        {
+                return compact_slot(flag, counter);
+        }
 }
 
 template <bool SHADOW_KERNEL>
@@ -213,26 +251,52 @@ struct ShadowView
         }
 };
 
+__device__ __forceinline__ uint32_t fast_div(const FastDiv& f, uint32_t n, uint32_t* rest)
+{
+        const uint32_t q = (uint32_t)(((unsigned long long)n * f.m) >> f.s);
+        *rest = n - q * f.d;
+        return q;
+}
+
 // paint_pixels: stratified jittered sample -> projector ray (painter.cpp:410-448,
 // sampler.h:26-64, engine.h:86-156)
 template <int N>
 __device__ __forceinline__ void raygen_one(const DevScene<N>& S, const PassDev& P, const PathView<N>& A, long long g,
                                            long long slot)
 {
-        const long long entry = g / P.spp_eff;
-        int s = (int)(g - entry * P.spp_eff);
-        const long long pixel = P.list ? P.list[entry] : entry;
+        long long entry, pixel;
+        int s;
+        int px[N - 1];
+        if (P.small)
+        {
+                uint32_t rest;
+                entry = fast_div(P.by_spp, (uint32_t)g, &rest);
+                s = (int)rest;
+                pixel = P.list ? P.list[entry] : entry;
+                uint32_t rem = (uint32_t)pixel;
+#pragma unroll
+                for (int j = 0; j < N - 1; ++j)
+                {
+                        rem = fast_div(P.by_screen[j], rem, &rest);
+                        px[j] = (int)rest;
+                }
+        }
+        else
+        {
+                entry = g / P.spp_eff;
+                s = (int)(g - entry * P.spp_eff);
+                pixel = P.list ? P.list[entry] : entry;
+                long long rem = pixel;
+#pragma unroll
+                for (int j = 0; j < N - 1; ++j)
+                {
+                        px[j] = (int)(rem % S.proj.screen[j]);
+                        rem /= S.proj.screen[j];
+                }
+        }
         long long sample = P.sample_offset + s;
         unsigned long long path = (unsigned long long)sample * (unsigned long long)P.npix + (unsigned long long)pixel;
 
-        int px[N - 1];
-        long long rem = pixel;
-#pragma unroll
-        for (int j = 0; j < N - 1; ++j)
-        {
-                px[j] = (int)(rem % S.proj.screen[j]);
-                rem /= S.proj.screen[j];
-        }
         float u[8];
         float4 a = rng4(P.key0, P.key1, path, 0, 0);
         u[0] = a.x;
@@ -245,12 +309,12 @@ __device__ __forceinline__ void raygen_one(const DevScene<N>& S, const PassDev& 
                 u[4] = b.x;
         }
         float point[N - 1];
-        int r = s;
+        uint32_t r = (uint32_t)s;
 #pragma unroll
         for (int j = 0; j < N - 1; ++j)
         {
-                int digit = r % P.k1d;
-                r /= P.k1d;
+                uint32_t digit;
+                r = fast_div(P.by_k, r, &digit);
                 float offset = __fdiv_rn((float)digit, (float)P.k1d);
                 float sample_j = offset + u[j] * P.recip_k;
                 point[j] = (float)px[j] + sample_j;
@@ -348,13 +412,13 @@ __device__ __forceinline__ void accumulate(double* accum, uint32_t pixel, float 
 // or an emitting hit adds its colour to the pixel; a diffuse hit emits one shadow ray per light into
 // the shadow queue and, below the depth cap, writes its continuation into the next path queue.
 template <int N>
-__global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_constant__ const DevScene<N> S, const PassDev P, PathView<N> A, HitView<N> H,
+__global__ void __launch_bounds__(BLOCK, shade_min_blocks<N>()) k_shade(__grid_constant__ const DevScene<N> S, const PassDev P, PathView<N> A, HitView<N> H,
                                                  PathView<N> B, ShadowView<N> SQ, ShadowView<N> SM, double* accum,
                                                  unsigned long long* counters, int parity)
 {
         const long long count = (long long)counters[C_Q_ACTIVE];
-        __shared__ int s_warp[BLOCK / 32];
-        __shared__ long long s_base;
+        __shared__ CompactShared s_compact;
+        int turn = 0;
         const bool one_mesh = S.nmesh == 1;
         long long shadow_rays = 0;  // shadow rays planned here (scenes with one mesh)
         const long long tiles = (count + blockDim.x - 1) / blockDim.x;
@@ -479,7 +543,7 @@ __global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_consta
                         }
                 }
 
-                // direct lighting: one shadow ray per light (block-uniform loop, compacted per light)
+                // direct lighting: one shadow ray per light (uniform loop, compacted per light)
                 for (int l = 0; l < S.nlights; ++l)
                 {
                         bool shadow = false;
@@ -557,7 +621,7 @@ __global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_consta
                                 }
                                 shadow = walk;
                         }
-                        long long qo = compact_slot(shadow, counters + C_SHADOW + parity, s_warp, &s_base);
+                        long long qo = shade_slot<N>(shadow, counters + C_SHADOW + parity, &s_compact, &turn);
                         if (shadow)
                         {
 #pragma unroll
@@ -575,8 +639,8 @@ __global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_consta
                         }
                         if (S.smooth_normal)
                         {
-                                // block-uniform: every thread of the block takes part in the compaction
-                                long long bo = compact_slot(behind, counters + C_SMOOTH + parity, s_warp, &s_base);
+                                // uniform: every thread of the block takes part in the compaction
+                                long long bo = shade_slot<N>(behind, counters + C_SMOOTH + parity, &s_compact, &turn);
                                 if (behind)
                                 {
 #pragma unroll
@@ -597,14 +661,30 @@ __global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_consta
                 // diffuse continuation (diffuse_lighting, painter.cpp:298-323)
                 bool survive = false;
                 float nr_org[N], nr_dir[N];
-                if (lit && level < S.max_depth)
+                const bool bounce = lit && level < S.max_depth;
+                unsigned long long path = 0;
+                if (bounce)
                 {
                         const unsigned long long px = P.moments ? pixel / (uint32_t)P.spp_eff
                                                                 : (P.list ? (unsigned long long)P.list[pixel] : pixel);
-                        unsigned long long path = (unsigned long long)sample * (unsigned long long)P.npix + px;
-                        float d[N];
-                        if (cosine_hemisphere<N>(P.key0, P.key1, path, (uint32_t)(1 + level), sn, d))
+                        path = (unsigned long long)sample * (unsigned long long)P.npix + px;
+                }
+                float ball[N - 1], len2 = 0;
+                bool sampled;
+                if constexpr (N >= 5)
+                {
+                        sampled = ball_point_warp<N>(bounce, P.key0, P.key1, path, (uint32_t)(1 + level), ball, &len2);
+                }
+                else
+                {
+                        sampled = !bounce || ball_point<N>(P.key0, P.key1, path, (uint32_t)(1 + level), ball, &len2);
+                }
+                if (sampled)
+                {
+                        if (bounce)
                         {
+                                float d[N];
+                                cosine_hemisphere<N>(ball, len2, sn, d);
                                 Ray<N> dr;
                                 ray_set<N>(dr, p, d);
                                 if (!(mesh && vdot<N>(dr.dir, gn) <= 0))
@@ -619,12 +699,12 @@ __global__ void __launch_bounds__(BLOCK, SHADE_MIN_BLOCKS) k_shade(__grid_consta
                                         }
                                 }
                         }
-                        else
-                        {
-                                err |= ERR_SAMPLING_LIMIT;
-                        }
                 }
-                long long so = compact_slot(survive, counters + C_ACTIVE_OUT, s_warp, &s_base);
+                else
+                {
+                        err |= ERR_SAMPLING_LIMIT;
+                }
+                long long so = shade_slot<N>(survive, counters + C_ACTIVE_OUT, &s_compact, &turn);
                 if (survive)
                 {
 #pragma unroll
@@ -767,32 +847,6 @@ __device__ __forceinline__ long long lane_refill(bool idle, unsigned long long* 
         return j < count ? j : -1;
 }
 
-// Appends this lane's queue index to a walk list when `walk` (one atomic per warp; the lanes of a warp
-// keep their order) and returns its list position (-1 without `walk`).  Every lane of the warp calls it.
-__device__ __forceinline__ long long list_append(bool walk, long long i, int* list, unsigned long long* count)
-{
-        const unsigned m = __ballot_sync(0xffffffffu, walk);
-        if (!m)
-        {
-                return -1;
-        }
-        const int lane = threadIdx.x & 31;
-        const int leader = __ffs(m) - 1;
-        unsigned long long base = 0;
-        if (lane == leader)
-        {
-                base = atomicAdd(count, (unsigned long long)__popc(m));
-        }
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (!walk)
-        {
-                return -1;
-        }
-        const long long q = (long long)base + __popc(m & lanemask_lt());
-        list[q] = (int)i;
-        return q;
-}
-
 static_assert(sizeof(ClosestPlan) <= 32, "a listed ray's plan takes 32 bytes");
 
 // Extension rays of a scene with one mesh, first pass: every ray's objects (closest_plan); the rays
@@ -839,9 +893,10 @@ __global__ void __launch_bounds__(BLOCK) k_plan_extend(__grid_constant__ const D
                                 }
                         }
                 }
-                const long long q = list_append(walk, i, list, counters + C_WALK_EXT);
+                const long long q = compact_slot(walk, counters + C_WALK_EXT);
                 if (q >= 0)
                 {
+                        list[q] = (int)i;
                         plans[q] = plan;
                 }
         }
@@ -868,37 +923,25 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
         ClosestPlan plan;
         while (true)
         {
-                // fill: every listed ray walks (the plan kernel finished the others), so one round fills
-                // every idle lane while rays remain
-                for (int round = 0; round < FILL_ROUNDS; ++round)
+                // every listed ray walks (the plan kernel finished the others)
+                const long long q = lane_refill(i < 0, counters + C_WORK_EXT, count, &exhausted);
+                if (q >= 0)
                 {
-                        const long long q = lane_refill(i < 0, counters + C_WORK_EXT, count, &exhausted);
-                        if (q >= 0)
-                        {
-                                const long long j = list[q];
-                                Ray<N> r;
+                        const long long j = list[q];
+                        Ray<N> r;
 #pragma unroll
-                                for (int k = 0; k < N; ++k)
-                                {
-                                        r.org[k] = A.at(k, j);
-                                        r.dir[k] = A.at(N + k, j);
-                                }
-                                plan = plans[q];  // listed rays have plan.walk set
-                                walk_begin<N>(M, w, r, plan.mesh_t, FLT_MAX);
-                                i = j;
-                        }
-                        if (exhausted || !__any_sync(0xffffffffu, i < 0))
+                        for (int k = 0; k < N; ++k)
                         {
-                                break;
+                                r.org[k] = A.at(k, j);
+                                r.dir[k] = A.at(N + k, j);
                         }
+                        plan = plans[q];  // listed rays have plan.walk set
+                        walk_begin<N>(M, w, r, plan.mesh_t, FLT_MAX);
+                        i = j;
                 }
                 if (!__any_sync(0xffffffffu, i >= 0))
                 {
-                        if (exhausted)
-                        {
-                                break;
-                        }
-                        continue;
+                        break;
                 }
                 {
                         float t = 0;
@@ -946,38 +989,25 @@ __global__ void __launch_bounds__(BLOCK, walk_min_blocks<N>())
         float dist = 0;
         while (true)
         {
-                for (int round = 0; round < FILL_ROUNDS; ++round)
+                const long long q = lane_refill(i < 0, counters + C_WORK_SH + parity, count, &exhausted);
+                if (q >= 0)
                 {
-                        const long long q = lane_refill(i < 0, counters + C_WORK_SH + parity, count, &exhausted);
-                        if (q >= 0)
-                        {
-                                const long long j = q;
-                                Ray<N> r;
+                        Ray<N> r;
 #pragma unroll
-                                for (int k = 0; k < N; ++k)
-                                {
-                                        r.org[k] = SQ.at(k, j);
-                                        r.dir[k] = SQ.at(N + k, j);
-                                }
-                                // queued by k_shade: nothing nearer than the light occludes it, and the mesh's
-                                // root box starts before the light at the stored entry distance
-                                const float dj = SQ.at(2 * N, j);
-                                walk_begin<N>(M, w, r, SQ.at(2 * N + 4, j), dj);
-                                dist = dj;
-                                i = j;
-                        }
-                        if (exhausted || !__any_sync(0xffffffffu, i < 0))
+                        for (int k = 0; k < N; ++k)
                         {
-                                break;
+                                r.org[k] = SQ.at(k, q);
+                                r.dir[k] = SQ.at(N + k, q);
                         }
+                        // queued by k_shade: nothing nearer than the light occludes it, and the mesh's
+                        // root box starts before the light at the stored entry distance
+                        dist = SQ.at(2 * N, q);
+                        walk_begin<N>(M, w, r, SQ.at(2 * N + 4, q), dist);
+                        i = q;
                 }
                 if (!__any_sync(0xffffffffu, i >= 0))
                 {
-                        if (exhausted)
-                        {
-                                break;
-                        }
-                        continue;
+                        break;
                 }
                 {
                         float t = 0;
@@ -1288,7 +1318,9 @@ const LaunchSizes& Wavefront<N>::prepare()
                 z.shadow_refill_blocks[1] = resident_blocks(k_shadow_refill<N, 1>, Stage<N, 1>::BYTES);
                 z.shadow_refill_blocks[2] = resident_blocks(k_shadow_refill<N, 2>, Stage<N, 2>::BYTES);
                 z.shadow_refill_blocks[3] = resident_blocks(k_shadow_refill<N, 4>, Stage<N, 4>::BYTES);
-                z.stream_blocks = resident_blocks(k_shade<N>);
+                z.raygen_blocks = resident_blocks(k_raygen<N>);
+                z.plan_blocks = resident_blocks(k_plan_extend<N>);
+                z.shade_blocks = resident_blocks(k_shade<N>);
                 return z;
         }();
         return sizes;
@@ -1308,14 +1340,15 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         const int vi = rounds < 0 ? 0 : (rounds >= 4 ? 3 : (rounds >= 2 ? 2 : 1));
         const long long extend_refill_blocks = L.extend_refill_blocks[vi];
         const long long shadow_refill_blocks = L.shadow_refill_blocks[vi];
-        const long long stream_blocks = L.stream_blocks;
         // scenes with exactly one mesh use the lane-refill walk kernels
         const bool one_mesh = S.nmesh == 1;
         const bool smooth = S.smooth_normal != 0;
         const long long walk_cap = std::max<long long>(1, (Q * lights + BLOCK - 1) / BLOCK);
         const unsigned ext_grid = (unsigned)std::min(one_mesh ? extend_refill_blocks : extend_blocks, walk_cap);
         const unsigned sh_grid = (unsigned)std::min(one_mesh ? shadow_refill_blocks : shadow_blocks, walk_cap);
-        const unsigned str_grid = (unsigned)std::min(stream_blocks * 2, walk_cap);
+        const unsigned raygen_grid = (unsigned)std::min(L.raygen_blocks, walk_cap);
+        const unsigned plan_grid = (unsigned)std::min(L.plan_blocks, walk_cap);
+        const unsigned shade_grid = (unsigned)std::min(L.shade_blocks, walk_cap);
         const bool flip = parity != 0;
         float* fa = flip ? fB : fA;
         float* fb = flip ? fA : fB;
@@ -1329,7 +1362,7 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         {
                 cudaEventRecord(ev[0], st);
         }
-        k_raygen<N><<<str_grid, BLOCK, 0, st>>>(S, P, A, counters);
+        k_raygen<N><<<raygen_grid, BLOCK, 0, st>>>(S, P, A, counters);
         if (ev)
         {
                 cudaEventRecord(ev[1], st);
@@ -1337,7 +1370,7 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         if (one_mesh)
         {
                 // rays that need no walk are finished by the plan kernel; the walk kernel takes the rest
-                k_plan_extend<N><<<str_grid, BLOCK, 0, st>>>(S, A, H, walk_ext, (ClosestPlan*)plan_ext, counters);
+                k_plan_extend<N><<<plan_grid, BLOCK, 0, st>>>(S, A, H, walk_ext, (ClosestPlan*)plan_ext, counters);
         }
         if (ev)
         {
@@ -1375,7 +1408,7 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
                 // the previous iteration's shadow walks read the queue that shading fills
                 cudaStreamWaitEvent(st, side->join, 0);
         }
-        k_shade<N><<<str_grid, BLOCK, 0, st>>>(S, P, A, H, B, SQ, SM, accum, counters, parity);
+        k_shade<N><<<shade_grid, BLOCK, 0, st>>>(S, P, A, H, B, SQ, SM, accum, counters, parity);
         if (ev)
         {
                 cudaEventRecord(ev[4], st);
@@ -1416,7 +1449,7 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         }
         if (smooth)
         {
-                k_shadow_smooth<N><<<str_grid, BLOCK, 0, sh>>>(S, SM, accum, counters, parity);
+                k_shadow_smooth<N><<<shade_grid, BLOCK, 0, sh>>>(S, SM, accum, counters, parity);
         }
         if (side)
         {

@@ -33,7 +33,10 @@ struct LaunchSizes
         // per walk variant: direct loads, then staging chunks of 1, 2, 4 rounds of 32 tests
         long long extend_refill_blocks[4] = {1, 1, 1, 1};
         long long shadow_refill_blocks[4] = {1, 1, 1, 1};
-        long long stream_blocks = 1;
+        // the streaming kernels: one wave of resident blocks each
+        long long raygen_blocks = 1;
+        long long plan_blocks = 1;
+        long long shade_blocks = 1;
 };
 
 // A second stream for the kernels of an iteration that the next one does not wait for, and the events that

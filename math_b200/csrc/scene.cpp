@@ -1453,6 +1453,35 @@ long long pass_first_sample(const nt_scene* s, const nt_render_opts& o)
         return o.sample_offset > 0 ? (long long)o.sample_offset : s->samples_done;
 }
 
+FastDiv fast_divisor(long long d)
+{
+        FastDiv f{1, 0x80000001u, 31};
+        if (d > 0 && d < (1ll << 31))
+        {
+                int l = 0;
+                while ((1ll << l) < d)
+                {
+                        ++l;
+                }
+                f.d = (uint32_t)d;
+                f.s = (uint32_t)(31 + l);
+                f.m = (uint32_t)((1ull << (31 + l)) / (unsigned long long)d + 1);
+        }
+        return f;
+}
+
+// The constants ray generation divides by (raygen_one).
+void set_divisors(PassDev* P, const nt_scene* s, long long total)
+{
+        P->small = total < (1ll << 31) && P->npix < (1ll << 31) ? 1 : 0;
+        P->by_spp = fast_divisor(P->spp_eff);
+        P->by_k = fast_divisor(P->k1d);
+        for (size_t j = 0; j < s->screen.size() && j < 5; ++j)
+        {
+                P->by_screen[j] = fast_divisor(s->screen[j]);
+        }
+}
+
 template <int N>
 std::unique_ptr<PassJob> prepare_pass(nt_scene* s, const nt_render_opts& o, const PassTarget& target = PassTarget())
 {
@@ -1524,6 +1553,7 @@ std::unique_ptr<PassJob> prepare_pass(nt_scene* s, const nt_render_opts& o, cons
         P.path_end = total;
         P.moments = moments_accum ? 1 : 0;
         P.list = target.list;
+        set_divisors(&P, s, total);
         if (moments_accum && total > 0xffffffffll)
         {
                 fail(NT_EINVAL, "too many paths in one moments pass");
@@ -1670,6 +1700,7 @@ void render_noalloc(nt_scene* s, const nt_render_opts& o, double* d_accum, long 
         P.sample_offset = sample_offset;
         P.path_begin = 0;
         P.path_end = total;
+        set_divisors(&P, s, total);
         check_cuda(cudaMemsetAsync(counters, 0, C_COUNT * sizeof(unsigned long long), st), "memset counters");
         unsigned long long host_counters[C_COUNT] = {};
         KernelTimes times;
