@@ -234,7 +234,7 @@ def measure_plain(scene, spec: dict, args, steps: int, rank: int, world: int, lo
     n = spec["n"]
     spp, depth = spec["spp"], spec["max_depth"]
     stream = torch.cuda.ExternalStream(scene.stream)
-    # the library's autotuner picks the path-pool size and the iterations per graph launch from probe
+    # the library's autotuner picks the path-pool size and the iterations between host checks from probe
     # passes of this frame (untimed; it clears the accumulator)
     tuned, _ = scene.autotune(spp, max_depth=depth, seed=spec["seed"])
     # every rank traces the same Philox stream; ranks take disjoint sample ranges (pass k of rank r
@@ -398,8 +398,8 @@ def measure_denoise(scene, n: int) -> dict:
 
 
 def run_batch(args) -> None:
-    """--config batch: the batched mixed workload (math_b200.batched): 64 seeded scenes of n = 3..6 in
-    one CUDA graph per pass (nt_render_batch), tuned per dimension by nt_autotune; wall clock around
+    """--config batch: the batched mixed workload (math_b200.batched): 64 seeded scenes of n = 3..6
+    side by side (nt_render_batch), tuned per dimension by nt_autotune; wall clock around
     each synchronous batch call; hull meshes cached under _build/meshes between runs."""
     from math_b200 import batched
 

@@ -75,8 +75,9 @@ typedef struct nt_render_opts
         int64_t pool_paths;     /* wavefront path pool size; <= 0: automatic */
         int timing;             /* 1: per-kernel CUDA-event times in nt_stats (iterations enqueued one by one) */
         const volatile int* stop; /* optional host stop flag, polled between batches of wavefront iterations */
-        int graph_iterations;   /* wavefront iterations per CUDA-graph launch (the host checks for the end of
-                                   the pass after each); <= 0: 4.  nt_autotune picks it with pool_paths. */
+        int graph_iterations;   /* wavefront iterations enqueued between the host's checks for the end of the
+                                   pass (rounded up to an even number); <= 0: 4.  nt_autotune picks it with
+                                   pool_paths. */
         int64_t sample_offset;  /* > 0: index of this pass's first sample per pixel (a sample range of its own,
                                    e.g. one rank's share of a frame rendered on several GPUs: samples
                                    [sample_offset, sample_offset + effective spp) trace the same paths whichever
@@ -261,13 +262,12 @@ int nt_accum_clear(nt_scene* scene);
 /* ---- batches and tuning (no counterpart in the reference, which paints one scene per call) ---- */
 
 /* One pass of each of `count` built scenes (distinct; any mix of dimensions), opts[i] for scene i,
- * run side by side: the wavefront iterations of all the passes, each on its scene's stream, are
- * captured into one CUDA graph, and the graph is launched until every pass has finished (a pass
- * that ends first idles through empty iterations).  stats: count entries, or NULL. */
+ * run side by side: opts[0].graph_iterations wavefront iterations of every unfinished pass are enqueued
+ * on its scene's streams in turn, until every pass has finished.  stats: count entries, or NULL. */
 int nt_render_batch(nt_scene* const* scenes, int count, const nt_render_opts* opts, nt_stats* stats);
 
 /* Times probe passes of `base` (its samples per pixel) over candidate path-pool sizes and iterations
- * per graph launch, then over the walk kernels' variants (walk_chunk 1, 32, 64, 128) and small-leaf
+ * between host checks, then over the walk kernels' variants (walk_chunk 1, 32, 64, 128) and small-leaf
  * thresholds (walk_small_leaf -1, 1, 2, 4) at the best of those, and returns the fastest in *tuned (a
  * copy of base with pool_paths, graph_iterations, walk_chunk and walk_small_leaf set) and its pass time
  * in *best_ms (may be NULL).  The probe passes go to the scene's

@@ -1,6 +1,6 @@
-"""The batched mixed workload: many scenes of mixed dimension and size rendered side by side in one
-CUDA graph (nt_render_batch), with per-dimension pool sizes and iterations per graph launch chosen by
-the autotuner (nt_autotune).
+"""The batched mixed workload: many scenes of mixed dimension and size rendered side by side
+(nt_render_batch), with per-dimension pool sizes and iterations between host checks chosen by the
+autotuner (nt_autotune).
 
     python -m math_b200.batched --scenes 64 --seed 0
 
@@ -8,7 +8,7 @@ Scenes: n uniform in {3, 4, 5, 6}; boundary of the convex hull of seeded points 
 point counts log-uniform in a per-dimension range; the floor, light and parallel camera of
 the measured scenes; screens log-uniform per dimension; 1 to 16 samples per pixel.  Prints one JSON
 line: paths/s of the batch, of the same passes rendered one after the other, and the tuned
-parameters per n (pool size, iterations per graph launch, walk staging chunk).
+parameters per n (pool size, iterations between host checks, walk staging chunk).
 """
 
 from __future__ import annotations

@@ -107,8 +107,7 @@ struct Wavefront
         }
 
         // The iteration kernels' attributes (dynamic shared memory of the walk kernels) and grid sizes,
-        // set up on the first call for this dimension.  Call it before capturing iterations into a
-        // graph (run() and the batch do).
+        // set up on the first call for this dimension.  Called before a pass's iterations are enqueued.
         static const LaunchSizes& prepare();
 };
 

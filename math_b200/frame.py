@@ -3,11 +3,11 @@
     python -m math_b200.frame --config n4 [--pool 33554432] [--iterations 8] [--frames 2] [--stats]
 
 The scene (`scenes.config`) is built with its trees on the GPU, then `--frames` frames of the
-configuration's sample count are rendered with the given pool size and iterations per graph launch
+configuration's sample count are rendered with the given pool size and iterations between host checks
 (the walk variant and small-leaf threshold are the library's defaults unless given).  With --stats the
 last frame is rendered with timing on, and its work counters and per-kernel event times are printed as
 one JSON line.  A profiler run over this command sees the tree build first (k_overlap, k_write,
-k_gather_records), then the frames' kernels in launch order: the first frame warms the graphs, so a
+k_gather_records), then the frames' kernels in launch order: the first frame warms the device, so a
 capture of the second frame's launches (skip the first frame's with the profiler's launch skip) shows
 the steady state.
 """
@@ -28,7 +28,7 @@ def main(argv=None) -> None:
     ap = argparse.ArgumentParser(description=__doc__.split("\n")[0])
     ap.add_argument("--config", default="n4", help="a scenes.config name (n3, n4, n5, n6, n4_small, ...)")
     ap.add_argument("--pool", type=int, default=1 << 25, help="paths in flight (pool_paths)")
-    ap.add_argument("--iterations", type=int, default=8, help="wavefront iterations per graph launch")
+    ap.add_argument("--iterations", type=int, default=8, help="wavefront iterations between host checks")
     ap.add_argument("--frames", type=int, default=2)
     ap.add_argument("--walk-chunk", type=int, default=0)
     ap.add_argument("--walk-small-leaf", type=int, default=0)

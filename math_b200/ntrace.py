@@ -234,7 +234,7 @@ def render_opts(samples_per_pixel: int, max_depth: int = 100, seed: int = 0, ret
 
 
 def render_batch(scenes: list, opts: list[dict]) -> list[dict]:
-    """One pass of each scene, run side by side in one CUDA graph (nt_render_batch); opts[i] holds
+    """One pass of each scene, run side by side (nt_render_batch); opts[i] holds
     the keyword arguments of Scene.render for scene i."""
     lib = library()
     n = len(scenes)
@@ -405,7 +405,7 @@ class Scene:
 
     def autotune(self, samples_per_pixel: int, max_depth: int = 100, seed: int = 0, retest: bool = True,
                  smooth_normal: bool = False) -> tuple[dict, float]:
-        """Fastest pool size, iterations per graph launch and walk staging chunk for passes of
+        """Fastest pool size, iterations between host checks and walk staging chunk for passes of
         samples_per_pixel (probe passes; clears the accumulator).  Returns ({pool_paths,
         graph_iterations, walk_chunk}, pass ms)."""
         base = render_opts(samples_per_pixel, max_depth, seed, retest, smooth_normal, 0, False, 0)
