@@ -20,6 +20,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace ntrace
@@ -38,9 +39,11 @@ constexpr int MAX_AXES = 5;
 // tap logits is GUIDE_SCALE x exp(min(o, BANDWIDTH_MAX)).
 constexpr int GUIDES = 3;
 constexpr float BANDWIDTH_MAX = 20.0f;
-// floats per pixel in the base-feature buffer: n + 10 of them used (n <= 6), the rest zero, so that a
-// pixel's features are four aligned 16-byte words
-constexpr int BASE_STRIDE = 16;
+// The base features of the pixels, as planes of float4 (plane g of pixel p at g x P + p), so that the
+// consecutive pixels of a warp read consecutive 16-byte words at every filter tap and stencil slot:
+//   0: mean (3), depth   1: standard deviation of the mean (3), spatial noise 0
+//   2: normal 0..3       3: spatial noise 1, 2, normal 4, 5
+constexpr int BASE_PLANES = 4;
 
 // ------------------------------------------------------------------------------------------------
 // tcgen05 GEMM
@@ -369,80 +372,138 @@ struct LoadCols
         }
 };
 
-// The screen and the network's feature stencil.
+// The screen and the network's feature stencil (at most 2^30 pixels, so 32-bit pixel numbers).
 struct Stencil
 {
         int axes;                   // n - 1
         int size[MAX_AXES];
-        long long stride[MAX_AXES];
+        unsigned stride[MAX_AXES];
         int nf;                     // base features per pixel
-        int stencil_features;       // nf x (2 axes + 1)
-        int features;               // stencil_features + 1: the noise level of the input last
+        int features;               // nf x (2 axes + 1) + 1: the noise level of the input last
+        unsigned pixels;
         float noise_level;          // 1 / sqrt(samples per pixel)
 
-        // pixel at offset d along axis a from p, clamped to the screen
-        __device__ __forceinline__ long long neighbour(long long p, int a, int d) const
+        // the pixel's position along axis a
+        __device__ __forceinline__ int position(unsigned p, int a) const
         {
-                const int x = (int)((p / stride[a]) % size[a]);
+                return (int)((p / stride[a]) % (unsigned)size[a]);
+        }
+        // pixel at offset d along axis a from p (at position x there), clamped to the screen
+        __device__ __forceinline__ unsigned neighbour(unsigned p, int a, int x, int d) const
+        {
                 const int y = min(max(x + d, 0), size[a] - 1);
-                return p + (long long)(y - x) * stride[a];
+                return (unsigned)((int)p + (y - x) * (int)stride[a]);
         }
 };
 
-// Source pixel of stencil slot q of pixel p (slot 0 the pixel, 2a + 1 / 2a + 2 its -1 / +1 neighbour
-// along axis a, clamped), in 32-bit arithmetic (at most 2^30 pixels)
-__device__ __forceinline__ unsigned slot_source(const Stencil& st, unsigned p, int q)
+struct Base
 {
-        if (q <= 0 || q > 2 * st.axes)
+        float4 g[BASE_PLANES];
+};
+
+// NS: the space dimension; planes a guide distance does not need are left out (FILTER: the normal's
+// fifth and sixth component share plane 3 with the spatial noise)
+template <int NS, bool FILTER>
+__device__ __forceinline__ void load_base(const float4* __restrict__ base, unsigned pixels, unsigned p, Base* b)
+{
+#pragma unroll
+        for (int g = 0; g < BASE_PLANES; ++g)
         {
-                return p;
+                if (!FILTER || g < 3 || NS > 4)
+                {
+                        b->g[g] = __ldg(base + (size_t)g * pixels + p);
+                }
         }
-        const int a = (q - 1) >> 1;
-        const unsigned stride = (unsigned)st.stride[a];
-        const int x = (int)((p / stride) % (unsigned)st.size[a]);
-        const int y = min(max(x + ((q & 1) ? -1 : 1), 0), st.size[a] - 1);
-        return (unsigned)((int)p + (y - x) * (int)stride);
 }
 
-// The network's input matrix X (pixels x padded features, BF16), written once per input: thread
-// (pixel, chunk) forms eight consecutive features and stores them as one 16-byte word, so that
-// consecutive threads write consecutive chunks of a row.  A chunk spans at most two stencil slots
-// (nf > 8), so the thread walks the slots incrementally: one source pixel per slot it touches.
-__global__ void k_features(long long P, __grid_constant__ const Stencil st, int Fp, const float* __restrict__ base, __nv_bfloat16* __restrict__ X)
+template <int NS>
+__device__ __forceinline__ float base_normal(const Base& b, int k)
 {
-        const int chunks = Fp / 8;
-        const long long total = P * chunks;
-        const int nf = st.nf;
-        const int S = 2 * st.axes + 1;
-        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
+        return k == 0 ? b.g[2].x : (k == 1 ? b.g[2].y : (k == 2 ? b.g[2].z : (k == 3 ? b.g[2].w : (k == 4 ? b.g[3].z : b.g[3].w))));
+}
+
+// Feature f of a stencil slot: mean (3), standard deviation (3), normal (NS), depth / 10, spatial noise (3)
+template <int NS>
+__device__ __forceinline__ float base_feature(const Base& b, int f)
+{
+        if (f < 3)
         {
-                const unsigned p = (unsigned)(i / chunks);
-                const int c = (int)(i - (long long)p * chunks);
-                int q = (c * 8) / nf;
-                int f = c * 8 - q * nf;
-                unsigned src = slot_source(st, p, q);
-                __align__(16) __nv_bfloat16 v[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
+                return f == 0 ? b.g[0].x : (f == 1 ? b.g[0].y : b.g[0].z);
+        }
+        if (f < 6)
+        {
+                return f == 3 ? b.g[1].x : (f == 4 ? b.g[1].y : b.g[1].z);
+        }
+        if (f < 6 + NS)
+        {
+                return base_normal<NS>(b, f - 6);
+        }
+        if (f == 6 + NS)
+        {
+                return b.g[0].w * 0.1f;
+        }
+        return f == 7 + NS ? b.g[1].w : (f == 8 + NS ? b.g[3].x : b.g[3].y);
+}
+
+// The network's padded input row of pixel p in BF16, eight consecutive features at a time: emit(chunk,
+// words).  Slot 0 is the pixel, slots 2a + 1 and 2a + 2 its -1 and +1 neighbours along axis a (clamped),
+// then the noise level and zeros.
+template <int NS, class Emit>
+__device__ __forceinline__ void feature_row(const Stencil& st, const float4* __restrict__ base, unsigned p, const Emit& emit)
+{
+        constexpr int NF = NS + 10;
+        constexpr int SLOTS = 2 * (NS - 1) + 1;
+        constexpr int F = NF * SLOTS + 1;
+        constexpr int FP = (F + 15) / 16 * 16;
+        __nv_bfloat162 w[4];
+        float even = 0;
+        int at = 0;
+        auto put = [&](float x) {
+                if (at & 1)
                 {
-                        float x = 0.0f;
-                        if (q < S)
+                        w[(at & 7) >> 1] = __floats2bfloat162_rn(even, x);
+                        if ((at & 7) == 7)
                         {
-                                x = __ldg(base + (size_t)src * BASE_STRIDE + f);
-                        }
-                        else if (q == S && f == 0)
-                        {
-                                x = st.noise_level;
-                        }
-                        v[j] = __float2bfloat16_rn(x);
-                        if (++f == nf)
-                        {
-                                f = 0;
-                                ++q;
-                                src = slot_source(st, p, q);
+                                emit(at >> 3, *reinterpret_cast<const uint4*>(w));
                         }
                 }
-                *reinterpret_cast<uint4*>(X + (size_t)p * Fp + c * 8) = *reinterpret_cast<const uint4*>(v);
+                even = x;
+                ++at;
+        };
+#pragma unroll
+        for (int q = 0; q < SLOTS; ++q)
+        {
+                unsigned src = p;
+                if (q > 0)
+                {
+                        const int a = (q - 1) >> 1;
+                        src = st.neighbour(p, a, st.position(p, a), (q & 1) ? -1 : 1);
+                }
+                Base b;
+                load_base<NS, false>(base, st.pixels, src, &b);
+#pragma unroll
+                for (int f = 0; f < NF; ++f)
+                {
+                        put(base_feature<NS>(b, f));
+                }
+        }
+        put(st.noise_level);
+#pragma unroll
+        for (int f = F; f < FP; ++f)
+        {
+                put(0.0f);
+        }
+}
+
+// The network's input matrix X (pixels x padded features, BF16), which training keeps.
+template <int NS>
+__global__ void k_features(__grid_constant__ const Stencil st, int Fp, const float4* __restrict__ base,
+                           __nv_bfloat16* __restrict__ X)
+{
+        for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < st.pixels; p += gridDim.x * blockDim.x)
+        {
+                uint4* row = reinterpret_cast<uint4*>(X + (size_t)p * Fp);
+                feature_row<NS>(st, base, p, [&](int c, uint4 v) { row[c] = v; });
         }
 }
 
@@ -462,25 +523,29 @@ struct EpiStoreF32
         }
 };
 
-// The epilogues below store a row's 16 columns as 16-byte words: out 16-byte aligned and ld a
-// multiple of 16 (every matrix they write has 64 or outputs_padded columns).
-struct EpiBiasF32
+// The output layer: column c of pixel `row` at c x rows + row (planes, so that the filter's consecutive
+// threads read consecutive words), the first `cols` columns only
+struct EpiBiasPlanes
 {
         const float* bias;
         float* out;
-        int ld;
+        int rows;
+        int cols;
         __device__ __forceinline__ void operator()(int row, int c0, const float* v) const
         {
-                float4* o = reinterpret_cast<float4*>(out + (size_t)row * ld + c0);
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                for (int j = 0; j < 16; ++j)
                 {
-                        o[j] = make_float4(v[4 * j] + bias[c0 + 4 * j], v[4 * j + 1] + bias[c0 + 4 * j + 1],
-                                           v[4 * j + 2] + bias[c0 + 4 * j + 2], v[4 * j + 3] + bias[c0 + 4 * j + 3]);
+                        if (c0 + j < cols)
+                        {
+                                out[(size_t)(c0 + j) * rows + row] = v[j] + bias[c0 + j];
+                        }
                 }
         }
 };
 
+// The epilogues below store a row's 16 columns as 16-byte words: out 16-byte aligned and ld a
+// multiple of 16 (every matrix they write has 64 columns).
 struct EpiBiasReluBF16
 {
         const float* bias;
@@ -590,60 +655,267 @@ cudaError_t gemm(const LA& la, const LB& lb, const EPI& epi, int M, int N, int K
 }
 
 // ------------------------------------------------------------------------------------------------
+// The whole network in one kernel, for inference
+//
+// The three layers as products of their own write and read the input matrix and both hidden layers
+// through memory (2.0 of the 3.2 GB an n = 4 frame of 2.1 M pixels moves).  Here a block keeps the
+// weights in shared memory and takes tiles of 128 pixels: each thread gathers its pixel's features into
+// the first layer's operand tile, and between the layers the accumulator goes from tensor memory through
+// bias, ReLU and BF16 rounding into the next one's operand tile; only the output planes are written.  The
+// phases of a tile follow each other; two or three blocks per SM (shared memory) fill each other's waits.
+// n = 4, 128^3 pixels: feature matrix and three products MLP_BEFORE ms -> MLP_AFTER ms.
+
+// K-major tile of K columns: core matrices of 8 rows x 16 bytes, K first
+__device__ __forceinline__ uint32_t tile_off_k(int K, int r, int c8)
+{
+        return (uint32_t)((r >> 3) * (K * 16) + c8 * 128 + (r & 7) * 16);
+}
+
+// D (tmem) = A B^T over K columns, both K-major tiles in shared memory; one thread issues
+__device__ __forceinline__ void mlp_mma(uint32_t tmem, uint32_t a, uint32_t b, int K, int N)
+{
+        const uint32_t idesc = umma_idesc_bf16(GM, N);
+        for (int s = 0; s < K / 16; ++s)
+        {
+                const uint64_t da = umma_desc(a + s * 256, 128, K * 16);
+                const uint64_t db = umma_desc(b + s * 256, 128, K * 16);
+                asm volatile(
+                        "{\n\t.reg .pred p;\n\t"
+                        "setp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+                        "l"(da), "l"(db), "r"(idesc), "r"(s > 0 ? 1u : 0u)
+                        : "memory");
+        }
+}
+
+template <int NS>
+struct MlpShape
+{
+        static constexpr int F = (NS + 10) * (2 * (NS - 1) + 1) + 1;
+        static constexpr int FP = (F + 15) / 16 * 16;
+        static constexpr int O = (TAPS + GUIDES) * (NS - 1);
+        static constexpr int OP = (O + 15) / 16 * 16;
+        // shared memory: the three weight tiles, the input tile, the hidden tile
+        static constexpr int W1 = 0;
+        static constexpr int W2 = W1 + HID * FP * 2;
+        static constexpr int W3 = W2 + HID * HID * 2;
+        static constexpr int X = W3 + OP * HID * 2;
+        static constexpr int H = X + GM * FP * 2;
+        static constexpr int BYTES = H + GM * HID * 2;
+        static constexpr int COLS = 64;  // tensor-memory columns (HID, OP <= 64)
+};
+
+__device__ __forceinline__ void mlp_weights(unsigned char* s, const __nv_bfloat16* __restrict__ w, int rows, int K)
+{
+        for (int i = threadIdx.x; i < rows * (K / 8); i += GTHREADS)
+        {
+                const int r = i / (K / 8), c = i - r * (K / 8);
+                *reinterpret_cast<uint4*>(s + tile_off_k(K, r, c)) = *reinterpret_cast<const uint4*>(w + (size_t)r * K + c * 8);
+        }
+}
+
+template <int NS>
+__global__ void __launch_bounds__(GTHREADS) k_mlp(__grid_constant__ const Stencil st, const float4* __restrict__ base,
+                                                  const __nv_bfloat16* __restrict__ W1, const float* __restrict__ b1,
+                                                  const __nv_bfloat16* __restrict__ W2, const float* __restrict__ b2,
+                                                  const __nv_bfloat16* __restrict__ W3, const float* __restrict__ b3,
+                                                  float* __restrict__ Z, int* err, const GemmCtl ctl)
+{
+        using M = MlpShape<NS>;
+        extern __shared__ __align__(1024) unsigned char g_smem[];
+        __shared__ __align__(8) unsigned long long s_bar;
+        __shared__ uint32_t s_tmem;
+        __shared__ float s_bias[2 * HID + M::OP];
+        const int tid = threadIdx.x;
+        const int warp = tid >> 5;
+        if (warp == 0)
+        {
+                asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                             "r"((uint32_t)M::COLS)
+                             : "memory");
+                asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+        if (tid == 0)
+        {
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_bar)) : "memory");
+                asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        mlp_weights(g_smem + M::W1, W1, HID, M::FP);
+        mlp_weights(g_smem + M::W2, W2, HID, HID);
+        mlp_weights(g_smem + M::W3, W3, M::OP, HID);
+        for (int i = tid; i < 2 * HID + M::OP; i += GTHREADS)
+        {
+                s_bias[i] = i < HID ? b1[i] : (i < 2 * HID ? b2[i - HID] : b3[i - 2 * HID]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tmem = s_tmem;
+        const uint32_t lanes = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's rows of the accumulator
+        const uint32_t sm = smem_u32(g_smem);
+        const unsigned tiles = (st.pixels + GM - 1) / GM;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (unsigned tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x)
+        {
+                const unsigned row = tile * GM + tid;
+                // rows past the end repeat the last pixel; they are not stored
+                feature_row<NS>(st, base, min(row, st.pixels - 1), [&](int c, uint4 v) {
+                        *reinterpret_cast<uint4*>(g_smem + M::X + tile_off_k(M::FP, tid, c)) = v;
+                });
+                for (int layer = 0; layer < 3 && ok; ++layer)
+                {
+                        // the operand tile is written (and the accumulator read) by all threads; the tensor
+                        // core reads shared memory through the async proxy
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncthreads();
+                        if (tid == 0 && !ctl.withhold)
+                        {
+                                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                                if (layer == 0)
+                                {
+                                        mlp_mma(tmem, sm + M::X, sm + M::W1, M::FP, HID);
+                                }
+                                else if (layer == 1)
+                                {
+                                        mlp_mma(tmem, sm + M::H, sm + M::W2, HID, HID);
+                                }
+                                else
+                                {
+                                        mlp_mma(tmem, sm + M::H, sm + M::W3, HID, M::OP);
+                                }
+                                asm volatile(
+                                        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                                smem_u32(&s_bar))
+                                        : "memory");
+                        }
+                        const bool done = mbar_wait(&s_bar, phase, ctl.wait_ns);
+                        phase ^= 1;
+                        ok = __syncthreads_and(done) != 0;
+                        if (!ok)
+                        {
+                                // once more before the accumulator is given back (bounded)
+                                mbar_wait(&s_bar, phase ^ 1, ctl.wait_ns);
+                                break;
+                        }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (layer < 2)
+                        {
+                                const float* bias = s_bias + layer * HID;
+#pragma unroll
+                                for (int c = 0; c < HID; c += 16)
+                                {
+                                        float v[16];
+                                        tmem_ld16(lanes + c, v);
+                                        __nv_bfloat162 h[8];
+#pragma unroll
+                                        for (int j = 0; j < 8; ++j)
+                                        {
+                                                h[j] = __floats2bfloat162_rn(fmaxf(v[2 * j] + bias[c + 2 * j], 0.0f),
+                                                                             fmaxf(v[2 * j + 1] + bias[c + 2 * j + 1], 0.0f));
+                                        }
+                                        unsigned char* dst = g_smem + M::H + tile_off_k(HID, tid, c / 8);
+                                        *reinterpret_cast<uint4*>(dst) = reinterpret_cast<const uint4*>(h)[0];
+                                        *reinterpret_cast<uint4*>(dst + 128) = reinterpret_cast<const uint4*>(h)[1];
+                                }
+                        }
+                        else
+                        {
+#pragma unroll
+                                for (int c = 0; c < M::OP; c += 16)
+                                {
+                                        float v[16];
+                                        tmem_ld16(lanes + c, v);
+                                        if (row < st.pixels)
+                                        {
+#pragma unroll
+                                                for (int j = 0; j < 16; ++j)
+                                                {
+                                                        if (c + j < M::O)
+                                                        {
+                                                                Z[(size_t)(c + j) * st.pixels + row] = v[j] + s_bias[2 * HID + c + j];
+                                                        }
+                                                }
+                                        }
+                                }
+                        }
+                }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        if (warp == 0)
+        {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)M::COLS) : "memory");
+        }
+        if (!ok && tid == 0 && err)
+        {
+                atomicOr(err, 1);
+        }
+}
+
+// ------------------------------------------------------------------------------------------------
 // CUDA-core kernels
 
 constexpr int TB = 256;
 
-unsigned blocks_for(long long n)
+unsigned blocks_for(long long n, int threads = TB)
 {
-        return (unsigned)std::min<long long>((n + TB - 1) / TB, 148LL * 64);
+        return (unsigned)std::min<long long>((n + threads - 1) / threads, 148LL * 64);
 }
 
-// per-pixel base features: mean (3), standard deviation of the mean (3), normal (n), depth / 10, and
-// the spatial noise estimate (3): sqrt of half the mean squared difference of the mean to the 2(n-1)
-// axis neighbours (clamped), which for independent noise over a locally constant image is the
-// standard deviation of the mean; unlike the per-pixel estimate it exists at one sample per pixel
-__global__ void k_base_features(long long P, __grid_constant__ const Stencil st, const float* __restrict__ mean, const float* __restrict__ var,
-                                const float* __restrict__ normal, const float* __restrict__ depth, float* __restrict__ out)
+// Threads per block of a kernel with one thread per pixel: small images take small blocks, so that they
+// spread over all SMs.
+int pixel_threads(long long P)
 {
-        const int nf = st.nf;
-        const int n = nf - 10;
-        const float inv = 1.0f / (float)(4 * st.axes);
-        for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x)
+        return P < 148LL * 2 * TB ? 64 : TB;
+}
+
+// The base-feature planes: mean, depth, standard deviation of the mean, normal, and the spatial noise
+// estimate: sqrt of half the mean squared difference of the mean to the 2(n-1) axis neighbours (clamped),
+// which for independent noise over a locally constant image is the standard deviation of the mean; unlike
+// the per-pixel estimate it exists at one sample per pixel.
+template <int NS>
+__global__ void k_base_features(__grid_constant__ const Stencil st, const float* __restrict__ mean, const float* __restrict__ var,
+                                const float* __restrict__ normal, const float* __restrict__ depth, float4* __restrict__ out)
+{
+        constexpr float INV = 1.0f / (float)(4 * (NS - 1));
+        for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < st.pixels; p += gridDim.x * blockDim.x)
         {
-                float* o = out + p * BASE_STRIDE;
-                float m[3], sq[3] = {0, 0, 0};
+                float m[3], sd[3], sq[3] = {0, 0, 0}, nv[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
                 for (int c = 0; c < 3; ++c)
                 {
-                        m[c] = mean[p * 3 + c];
-                        o[c] = m[c];
-                        o[3 + c] = sqrtf(fmaxf(var[p * 3 + c], 0.0f));
+                        m[c] = mean[(size_t)p * 3 + c];
+                        sd[c] = sqrtf(fmaxf(var[(size_t)p * 3 + c], 0.0f));
                 }
-                for (int k = 0; k < n; ++k)
+#pragma unroll
+                for (int k = 0; k < NS; ++k)
                 {
-                        o[6 + k] = normal[p * n + k];
+                        nv[k] = normal[(size_t)p * NS + k];
                 }
-                o[6 + n] = depth[p] * 0.1f;
-                for (int a = 0; a < st.axes; ++a)
+#pragma unroll
+                for (int a = 0; a < NS - 1; ++a)
                 {
+                        const int x = st.position(p, a);
+#pragma unroll
                         for (int d = -1; d <= 1; d += 2)
                         {
-                                const long long q = st.neighbour(p, a, d);
+                                const unsigned q = st.neighbour(p, a, x, d);
+#pragma unroll
                                 for (int c = 0; c < 3; ++c)
                                 {
-                                        const float t = mean[q * 3 + c] - m[c];
+                                        const float t = mean[(size_t)q * 3 + c] - m[c];
                                         sq[c] += t * t;
                                 }
                         }
                 }
-                for (int c = 0; c < 3; ++c)
-                {
-                        o[7 + n + c] = sqrtf(sq[c] * inv);
-                }
-                for (int k = nf; k < BASE_STRIDE; ++k)
-                {
-                        o[k] = 0.0f;
-                }
+                const size_t P = st.pixels;
+                out[p] = make_float4(m[0], m[1], m[2], depth[p]);
+                out[P + p] = make_float4(sd[0], sd[1], sd[2], sqrtf(sq[0] * INV));
+                out[2 * P + p] = make_float4(nv[0], nv[1], nv[2], nv[3]);
+                out[3 * P + p] = make_float4(sqrtf(sq[1] * INV), sqrtf(sq[2] * INV), nv[4], nv[5]);
         }
 }
 
@@ -677,160 +949,158 @@ __device__ __forceinline__ float guide_scale(int g)
         return g == 0 ? 4.0f : (g == 1 ? 1.0f : 0.05f);
 }
 
-// Guide distances between pixels p and q from the base features (mean 0..2, standard deviation of the
-// mean 3..5, normal 6..6+n-1, depth / 10 at 6+n, spatial noise 7+n..9+n): squared normal difference, squared depth
-// difference, and the colour distance of non-local-means filtering (Rousselle, Knaus and Zwicker,
-// "Adaptive rendering with non-local means filtering", 2012): the squared difference of the means
-// less the variance it carries from the noise, over that variance plus a small relative floor,
-// averaged over the channels.
-__device__ __forceinline__ void load_base(const float* __restrict__ base, long long p, float* b)
-{
-        const float4* s = reinterpret_cast<const float4*>(base + p * BASE_STRIDE);
-#pragma unroll
-        for (int i = 0; i < BASE_STRIDE / 4; ++i)
-        {
-                const float4 t = __ldg(s + i);
-                b[4 * i] = t.x;
-                b[4 * i + 1] = t.y;
-                b[4 * i + 2] = t.z;
-                b[4 * i + 3] = t.w;
-        }
-}
-
-// bp, bq: the two pixels' base features (load_base); n: the space dimension (3..6)
-__device__ __forceinline__ void guide_distance(const float* bp, const float* bq, int n, float* D)
+// Guide distances between two pixels: squared normal difference, squared depth difference, and the colour
+// distance of non-local-means filtering (Rousselle, Knaus and Zwicker, "Adaptive rendering with non-local
+// means filtering", 2012): the squared difference of the means less the variance it carries from the
+// noise, over that variance plus a small relative floor, averaged over the channels.  (The three
+// quotients by the fast divide, 2 ulp: the distances weigh logits that come out of BF16 products.)
+template <int NS>
+__device__ __forceinline__ void guide_distance(const Base& bp, const Base& bq, float* D)
 {
         float dn = 0;
 #pragma unroll
-        for (int k = 0; k < 6; ++k)
+        for (int k = 0; k < NS; ++k)
         {
-                if (k < n)
-                {
-                        const float t = bp[6 + k] - bq[6 + k];
-                        dn += t * t;
-                }
+                const float t = base_normal<NS>(bp, k) - base_normal<NS>(bq, k);
+                dn += t * t;
         }
-        // depth / 10 at 6 + n, picked by selects (an index computed from n would send the arrays to
-        // local memory)
-        const float dp = n == 3 ? bp[9] : (n == 4 ? bp[10] : (n == 5 ? bp[11] : bp[12]));
-        const float dq = n == 3 ? bq[9] : (n == 4 ? bq[10] : (n == 5 ? bq[11] : bq[12]));
-        const float dd = 10.0f * (dp - dq);
+        const float dd = bp.g[0].w - bq.g[0].w;
+        const float pm[3] = {bp.g[0].x, bp.g[0].y, bp.g[0].z}, qm[3] = {bq.g[0].x, bq.g[0].y, bq.g[0].z};
+        const float ps[3] = {bp.g[1].x, bp.g[1].y, bp.g[1].z}, qs[3] = {bq.g[1].x, bq.g[1].y, bq.g[1].z};
         float dc = 0;
 #pragma unroll
         for (int c = 0; c < 3; ++c)
         {
-                const float dm = bp[c] - bq[c];
-                const float v = bp[3 + c] * bp[3 + c] + bq[3 + c] * bq[3 + c];
-                const float mb = 0.5f * (bp[c] + bq[c]);
-                dc += fmaxf(dm * dm - v, 0.0f) / (1e-4f + 0.01f * mb * mb + v);
+                const float dm = pm[c] - qm[c];
+                const float v = ps[c] * ps[c] + qs[c] * qs[c];
+                const float mb = 0.5f * (pm[c] + qm[c]);
+                dc += __fdividef(fmaxf(dm * dm - v, 0.0f), 1e-4f + 0.01f * mb * mb + v);
         }
         D[0] = dn;
         D[1] = dd * dd;
         D[2] = dc * (1.0f / 3.0f);
 }
 
-// The axis's tap weights at pixel p: softmax over taps of Z[p, a*9 + j] - sum_g s_g D_g(p, tap j),
-// s_g = GUIDE_SCALE x exp(min(Z[p, 9 (n-1) + a*3 + g], BANDWIDTH_MAX)).  The taps' pixels q, D, s and
+// The axis's tap weights at pixel p: softmax over taps of Z[a*9 + j, p] - sum_g s_g D_g(p, tap j),
+// s_g = GUIDE_SCALE x exp(min(Z[9 (n-1) + a*3 + g, p], BANDWIDTH_MAX)).  The taps' pixels q, D, s and
 // whether each log-bandwidth lies below its clamp are returned for the backward pass.
-__device__ __forceinline__ void tap_weights(const Stencil& st, const float* __restrict__ base, int a, long long p,
-                                            const float* __restrict__ Z, int ldz, long long* q, float (*D)[GUIDES],
-                                            float* s, bool* open, float* w)
+template <int NS>
+__device__ __forceinline__ void tap_weights(const Stencil& st, const float4* __restrict__ base, int a, unsigned p,
+                                            const float* __restrict__ Z, unsigned* q, float (*D)[GUIDES], float* s,
+                                            bool* open, float* w)
 {
-        const float* zrow = Z + p * ldz;
+        const size_t P = st.pixels;
 #pragma unroll
         for (int g = 0; g < GUIDES; ++g)
         {
-                const float o = zrow[st.axes * TAPS + a * GUIDES + g];
+                const float o = __ldg(Z + (size_t)((NS - 1) * TAPS + a * GUIDES + g) * P + p);
                 open[g] = o < BANDWIDTH_MAX;
                 s[g] = guide_scale(g) * expf(fminf(o, BANDWIDTH_MAX));
         }
         float z[TAPS];
-        float bp[BASE_STRIDE];
-        load_base(base, p, bp);
+        Base bp;
+        load_base<NS, true>(base, st.pixels, p, &bp);
+        const int x = st.position(p, a);
 #pragma unroll
         for (int j = 0; j < TAPS; ++j)
         {
-                q[j] = st.neighbour(p, a, j - RADIUS);
-                float bq[BASE_STRIDE];
-                load_base(base, q[j], bq);
-                guide_distance(bp, bq, st.nf - 10, D[j]);
-                z[j] = zrow[a * TAPS + j] - (s[0] * D[j][0] + s[1] * D[j][1] + s[2] * D[j][2]);
+                q[j] = st.neighbour(p, a, x, j - RADIUS);
+                z[j] = __ldg(Z + (size_t)(a * TAPS + j) * P + p);
+                if (j == RADIUS)
+                {
+                        // the pixel itself
+                        D[j][0] = D[j][1] = D[j][2] = 0.0f;
+                        continue;
+                }
+                Base bq;
+                load_base<NS, true>(base, st.pixels, q[j], &bq);
+                guide_distance<NS>(bp, bq, D[j]);
+                z[j] -= s[0] * D[j][0] + s[1] * D[j][1] + s[2] * D[j][2];
         }
         softmax9(z, w);
 }
 
-// y_out[p] = sum_j w_j y_in[p + (j - 4) e_a] with the tap weights above
-__global__ void k_filter_fwd(long long P, __grid_constant__ const Stencil st, int a, const float* __restrict__ base, const float* __restrict__ Z,
-                             int ldz, const float* __restrict__ y_in, float* __restrict__ y_out)
+// y_out[p] = sum_j w_j y_in[p + (j - 4) e_a] with the tap weights above; images as float4 per pixel (the
+// input image is base plane 0), the last axis's result as three floats per pixel in out3 when given.
+// Bound by its instructions (about 700 per pixel and axis) with float4 planes: the base features as 64-byte
+// rows per pixel and 64-bit pixel arithmetic took FILTER_BEFORE us per pass over 128^3 pixels, this FILTER_AFTER.
+template <int NS>
+__global__ void k_filter_fwd(__grid_constant__ const Stencil st, int a, const float4* __restrict__ base,
+                             const float* __restrict__ Z, const float4* __restrict__ y_in, float4* __restrict__ y_out,
+                             float* __restrict__ out3)
 {
-        for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x)
+        for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < st.pixels; p += gridDim.x * blockDim.x)
         {
-                long long q[TAPS];
+                unsigned q[TAPS];
                 float D[TAPS][GUIDES], s[GUIDES], w[TAPS];
                 bool open[GUIDES];
-                tap_weights(st, base, a, p, Z, ldz, q, D, s, open, w);
+                tap_weights<NS>(st, base, a, p, Z, q, D, s, open, w);
                 float acc[3] = {0, 0, 0};
 #pragma unroll
                 for (int j = 0; j < TAPS; ++j)
                 {
-#pragma unroll
-                        for (int c = 0; c < 3; ++c)
-                        {
-                                acc[c] += w[j] * y_in[q[j] * 3 + c];
-                        }
+                        const float4 y = __ldg(y_in + q[j]);
+                        acc[0] += w[j] * y.x;
+                        acc[1] += w[j] * y.y;
+                        acc[2] += w[j] * y.z;
                 }
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
+                if (out3)
                 {
-                        y_out[p * 3 + c] = acc[c];
+                        out3[(size_t)p * 3] = acc[0];
+                        out3[(size_t)p * 3 + 1] = acc[1];
+                        out3[(size_t)p * 3 + 2] = acc[2];
+                }
+                else
+                {
+                        y_out[p] = make_float4(acc[0], acc[1], acc[2], 0.0f);
                 }
         }
 }
 
 // backward of k_filter_fwd: dZ for the axis's tap logits and log-bandwidths (through the softmax) and,
-// when g_in is given, dL/dy_in added by atomics
-__global__ void k_filter_bwd(long long P, __grid_constant__ const Stencil st, int a, const float* __restrict__ base, const float* __restrict__ Z,
-                             int ldz, const float* __restrict__ y_in, const float* __restrict__ g_out, float* g_in,
-                             __nv_bfloat16* __restrict__ dZ)
+// when g_in is given, dL/dy_in added by atomics (four floats at a time)
+template <int NS>
+__global__ void k_filter_bwd(__grid_constant__ const Stencil st, int a, const float4* __restrict__ base,
+                             const float* __restrict__ Z, const float4* __restrict__ y_in, const float4* __restrict__ g_out,
+                             float4* g_in, int ldz, __nv_bfloat16* __restrict__ dZ)
 {
-        for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x)
+        for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < st.pixels; p += gridDim.x * blockDim.x)
         {
-                long long q[TAPS];
+                unsigned q[TAPS];
                 float D[TAPS][GUIDES], s[GUIDES], w[TAPS], dw[TAPS];
                 bool open[GUIDES];
-                tap_weights(st, base, a, p, Z, ldz, q, D, s, open, w);
-                const float g0 = g_out[p * 3], g1 = g_out[p * 3 + 1], g2 = g_out[p * 3 + 2];
+                tap_weights<NS>(st, base, a, p, Z, q, D, s, open, w);
+                const float4 g = g_out[p];
                 float dot = 0;
 #pragma unroll
                 for (int j = 0; j < TAPS; ++j)
                 {
-                        const long long qj = q[j];
-                        dw[j] = g0 * y_in[qj * 3] + g1 * y_in[qj * 3 + 1] + g2 * y_in[qj * 3 + 2];
+                        const float4 y = __ldg(y_in + q[j]);
+                        dw[j] = g.x * y.x + g.y * y.y + g.z * y.z;
                         dot += w[j] * dw[j];
                         if (g_in)
                         {
-                                atomicAdd(g_in + qj * 3, w[j] * g0);
-                                atomicAdd(g_in + qj * 3 + 1, w[j] * g1);
-                                atomicAdd(g_in + qj * 3 + 2, w[j] * g2);
+                                atomicAdd(g_in + q[j], make_float4(w[j] * g.x, w[j] * g.y, w[j] * g.z, 0.0f));
                         }
                 }
                 float ds[GUIDES] = {0, 0, 0};
+                __nv_bfloat16* row = dZ + (size_t)p * ldz;
 #pragma unroll
                 for (int j = 0; j < TAPS; ++j)
                 {
                         const float gl = w[j] * (dw[j] - dot);
-                        dZ[p * ldz + a * TAPS + j] = __float2bfloat16_rn(gl);
+                        row[a * TAPS + j] = __float2bfloat16_rn(gl);
 #pragma unroll
-                        for (int g = 0; g < GUIDES; ++g)
+                        for (int k = 0; k < GUIDES; ++k)
                         {
-                                ds[g] -= gl * D[j][g];
+                                ds[k] -= gl * D[j][k];
                         }
                 }
                 // d logit_j / d o_g = -s_g D_g(j), zero where the log-bandwidth is clamped
 #pragma unroll
-                for (int g = 0; g < GUIDES; ++g)
+                for (int k = 0; k < GUIDES; ++k)
                 {
-                        dZ[p * ldz + st.axes * TAPS + a * GUIDES + g] = __float2bfloat16_rn(open[g] ? ds[g] * s[g] : 0.0f);
+                        row[(NS - 1) * TAPS + a * GUIDES + k] = __float2bfloat16_rn(open[k] ? ds[k] * s[k] : 0.0f);
                 }
         }
 }
@@ -859,15 +1129,23 @@ __device__ __forceinline__ double block_sum(double v, double* s_red)
         return t;
 }
 
+__device__ __forceinline__ double square_error(const float4 y, const float* __restrict__ target, unsigned p, double* d)
+{
+        d[0] = (double)y.x - (double)target[(size_t)p * 3];
+        d[1] = (double)y.y - (double)target[(size_t)p * 3 + 1];
+        d[2] = (double)y.z - (double)target[(size_t)p * 3 + 2];
+        return d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+}
+
 // sums[0] += sum((noisy - target)^2), the squared error of the input
-__global__ void k_energy(long long n3, const float* __restrict__ noisy, const float* __restrict__ target, double* sums)
+__global__ void k_energy(unsigned P, const float4* __restrict__ noisy, const float* __restrict__ target, double* sums)
 {
         __shared__ double s_red[TB / 32];
         double acc = 0;
-        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n3; i += (long long)gridDim.x * blockDim.x)
+        for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x)
         {
-                const double t = (double)noisy[i] - (double)target[i];
-                acc += t * t;
+                double d[3];
+                acc += square_error(noisy[p], target, p, d);
         }
         const double b = block_sum(acc, s_red);
         if (threadIdx.x == 0)
@@ -877,17 +1155,17 @@ __global__ void k_energy(long long n3, const float* __restrict__ noisy, const fl
 }
 
 // sums[1] += sum((out - target)^2) / sums[0]; g = 2 (out - target) / sums[0]
-__global__ void k_loss_grad(long long n3, const float* __restrict__ out, const float* __restrict__ target, double* sums,
-                            float* __restrict__ g)
+__global__ void k_loss_grad(unsigned P, const float4* __restrict__ out, const float* __restrict__ target, double* sums,
+                            float4* __restrict__ g)
 {
         __shared__ double s_red[TB / 32];
         const double inv = sums[0] > 0 ? 1.0 / sums[0] : 0.0;
         double acc = 0;
-        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n3; i += (long long)gridDim.x * blockDim.x)
+        for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x)
         {
-                const double d = (double)out[i] - (double)target[i];
-                acc += d * d;
-                g[i] = (float)(2.0 * d * inv);
+                double d[3];
+                acc += square_error(out[p], target, p, d);
+                g[p] = make_float4((float)(2.0 * d[0] * inv), (float)(2.0 * d[1] * inv), (float)(2.0 * d[2] * inv), 0.0f);
         }
         const double b = block_sum(acc, s_red);
         if (threadIdx.x == 0)
@@ -896,22 +1174,44 @@ __global__ void k_loss_grad(long long n3, const float* __restrict__ out, const f
         }
 }
 
-// out[c] += sum over rows of m[row, c] (c < cols)
-__global__ void k_colsum(long long rows, int cols, int ld, const __nv_bfloat16* __restrict__ m, float* out)
+// The bias gradients: out[c] += sum over rows of m[row, c] (c < cols), for the three layers' matrices at
+// once (blockIdx.y).  A block sums its rows in shared memory and adds each column once: with an addition
+// per thread group the three sums took 16 to 20 us each over 13,824 rows (262,144 atomics on 64
+// addresses).
+struct ColSums
 {
+        const __nv_bfloat16* m[3];
+        float* out[3];
+        int cols[3];
+};
+
+__global__ void __launch_bounds__(TB) k_colsum(long long rows, const ColSums cs)
+{
+        __shared__ float s_sum[TB];
+        const __nv_bfloat16* const m = cs.m[blockIdx.y];
+        const int cols = cs.cols[blockIdx.y];  // also the row length
         const int c = threadIdx.x % 64;
         const int rg = threadIdx.x / 64;
-        const int groups = blockDim.x / 64;
-        if (c >= cols)
-        {
-                return;
-        }
         float acc = 0;
-        for (long long r = blockIdx.x * (long long)groups + rg; r < rows; r += (long long)gridDim.x * groups)
+        if (c < cols)
         {
-                acc += __bfloat162float(m[r * ld + c]);
+                for (long long r = blockIdx.x * (long long)(TB / 64) + rg; r < rows; r += (long long)gridDim.x * (TB / 64))
+                {
+                        acc += __bfloat162float(m[r * cols + c]);
+                }
         }
-        atomicAdd(out + c, acc);
+        s_sum[threadIdx.x] = acc;
+        __syncthreads();
+        if (threadIdx.x < cols && threadIdx.x < 64)
+        {
+                float t = 0;
+#pragma unroll
+                for (int k = 0; k < TB / 64; ++k)
+                {
+                        t += s_sum[k * 64 + threadIdx.x];
+                }
+                atomicAdd(cs.out[blockIdx.y] + threadIdx.x, t);
+        }
 }
 
 __global__ void k_adam(long long count, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
@@ -1115,9 +1415,14 @@ struct nt_denoiser
         // padded FP32 gradients in one block (cleared together): gW1 | gb1 | gW2 | gb2 | gW3 | gb3
         Buf gblock;
         float *gW1 = nullptr, *gb1 = nullptr, *gW2 = nullptr, *gb2 = nullptr, *gW3 = nullptr, *gb3 = nullptr;
-        // per-image workspace
-        Buf base, X, H1, H2, Z, Y, G, dZ, dH1, dH2, sums, err;
+        // per-image workspace, one allocation for inference and one more for training, carved for the
+        // current image (set_input, forward)
+        Buf infer_ws, train_ws, sums, err;
+        float4 *base = nullptr, *Y = nullptr, *G = nullptr;
+        float* Z = nullptr;
+        __nv_bfloat16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dZ = nullptr, *dH1 = nullptr, *dH2 = nullptr;
         bool packed = false;
+        bool features = false;  // X holds the current input's feature matrix
 
         size_t gbytes() const
         {
@@ -1147,8 +1452,7 @@ void check_err(nt_denoiser* d)
         }
 }
 
-// forward pass of the current input: Y[n-1] is the denoised image
-void forward(nt_denoiser* d)
+void check_input(nt_denoiser* d)
 {
         if (d->P <= 0)
         {
@@ -1158,63 +1462,128 @@ void forward(nt_denoiser* d)
         {
                 pack(d);
         }
-        const long long P = d->P;
-        const int P32 = (int)P;
-        cudaStream_t s = d->st_use;
-        int* err = d->err.as<int>();
-        ck(gemm(LoadRows{d->X.as<__nv_bfloat16>(), d->Fp}, LoadRows{d->W1.as<__nv_bfloat16>(), d->Fp},
-                EpiBiasReluBF16{d->b1.as<float>(), d->H1.as<__nv_bfloat16>(), HID}, P32, HID, d->Fp, 0, err, s),
-           "gemm 1");
-        ck(gemm(LoadRows{d->H1.as<__nv_bfloat16>(), HID}, LoadRows{d->W2.as<__nv_bfloat16>(), HID},
-                EpiBiasReluBF16{d->b2.as<float>(), d->H2.as<__nv_bfloat16>(), HID}, P32, HID, HID, 0, err, s),
-           "gemm 2");
-        ck(gemm(LoadRows{d->H2.as<__nv_bfloat16>(), HID}, LoadRows{d->W3.as<__nv_bfloat16>(), HID},
-                EpiBiasF32{d->b3.as<float>(), d->Z.as<float>(), d->Op}, P32, d->Op, HID, 0, err, s),
-           "gemm 3");
-        for (int a = 0; a < d->n - 1; ++a)
+}
+
+// image a of the filter chain: 0 the noisy mean (base plane 0), a the result of axis a - 1
+float4* image(nt_denoiser* d, int a)
+{
+        return a == 0 ? d->base : d->Y + (size_t)(a - 1) * d->P;
+}
+
+// the filter passes over the output planes Z; the last one writes out3 when given
+template <int NS>
+void filter(nt_denoiser* d, float* out3)
+{
+        const int tb = pixel_threads(d->P);
+        for (int a = 0; a < NS - 1; ++a)
         {
-                k_filter_fwd<<<blocks_for(P), TB, 0, s>>>(P, d->st, a, d->base.as<float>(), d->Z.as<float>(), d->Op,
-                                                            d->Y.as<float>() + (size_t)a * P * 3,
-                                                            d->Y.as<float>() + (size_t)(a + 1) * P * 3);
+                k_filter_fwd<NS><<<blocks_for(d->P, tb), tb, 0, d->st_use>>>(d->st, a, d->base, d->Z,
+                                                                             image(d, a), image(d, a + 1),
+                                                                             a == NS - 2 ? out3 : nullptr);
         }
         ck(cudaGetLastError(), "filter");
 }
 
+// inference: the denoised image into d_out
+template <int NS>
+void infer(nt_denoiser* d, float* d_out)
+{
+        using M = MlpShape<NS>;
+        check_input(d);
+        int dev = 0, sms = 148;
+        ck(cudaGetDevice(&dev), "device");
+        ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
+        ck(cudaFuncSetAttribute(k_mlp<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::BYTES), "shared memory");
+        // as many blocks as fit an SM's shared memory (two or three: never more than its tensor memory holds)
+        const int per_sm = SM_SMEM / (M::BYTES + 2560);
+        static_assert(SM_SMEM / (M::BYTES + 2560) >= 1 && SM_SMEM / (M::BYTES + 2560) <= 512 / M::COLS);
+        const long long resident = (long long)std::max(1, sms) * per_sm;
+        const long long tiles = (d->P + GM - 1) / GM;
+        k_mlp<NS><<<(unsigned)std::min<long long>(tiles, resident), GTHREADS, M::BYTES, d->st_use>>>(
+                d->st, d->base, d->W1.as<__nv_bfloat16>(), d->b1.as<float>(), d->W2.as<__nv_bfloat16>(),
+                d->b2.as<float>(), d->W3.as<__nv_bfloat16>(), d->b3.as<float>(), d->Z, d->err.as<int>(), GemmCtl{});
+        ck(cudaGetLastError(), "network");
+        filter<NS>(d, d_out);
+}
+
+// forward pass of training: keeps the feature matrix, the hidden layers and the images
+template <int NS>
+void forward(nt_denoiser* d)
+{
+        check_input(d);
+        const long long P = d->P;
+        const int P32 = (int)P;
+        cudaStream_t s = d->st_use;
+        int* err = d->err.as<int>();
+        if (!d->X)
+        {
+                auto size = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+                const size_t half = sizeof(__nv_bfloat16) * (size_t)P;
+                const size_t xb = size(half * d->Fp), hb = size(half * HID), zb = size(half * d->Op);
+                const size_t gb = size(sizeof(float4) * (size_t)P * 2);
+                d->train_ws.ensure(xb + 4 * hb + zb + gb);
+                char* w = d->train_ws.as<char>();
+                d->X = (__nv_bfloat16*)w;
+                d->H1 = (__nv_bfloat16*)(w + xb);
+                d->H2 = (__nv_bfloat16*)(w + xb + hb);
+                d->dH1 = (__nv_bfloat16*)(w + xb + 2 * hb);
+                d->dH2 = (__nv_bfloat16*)(w + xb + 3 * hb);
+                d->dZ = (__nv_bfloat16*)(w + xb + 4 * hb);
+                d->G = (float4*)(w + xb + 4 * hb + zb);
+                // the padding columns of dZ are never written: cleared once per image
+                ck(cudaMemsetAsync(d->dZ, 0, zb, s), "memset");
+        }
+        if (!d->features)
+        {
+                const int tb = pixel_threads(P);
+                k_features<NS><<<blocks_for(P, tb), tb, 0, s>>>(d->st, d->Fp, d->base, d->X);
+                ck(cudaGetLastError(), "features");
+                d->features = true;
+        }
+        ck(gemm(LoadRows{d->X, d->Fp}, LoadRows{d->W1.as<__nv_bfloat16>(), d->Fp},
+                EpiBiasReluBF16{d->b1.as<float>(), d->H1, HID}, P32, HID, d->Fp, 0, err, s),
+           "gemm 1");
+        ck(gemm(LoadRows{d->H1, HID}, LoadRows{d->W2.as<__nv_bfloat16>(), HID},
+                EpiBiasReluBF16{d->b2.as<float>(), d->H2, HID}, P32, HID, HID, 0, err, s),
+           "gemm 2");
+        ck(gemm(LoadRows{d->H2, HID}, LoadRows{d->W3.as<__nv_bfloat16>(), HID},
+                EpiBiasPlanes{d->b3.as<float>(), d->Z, P32, d->O}, P32, d->Op, HID, 0, err, s),
+           "gemm 3");
+        filter<NS>(d, nullptr);
+}
+
 // loss and gradients (padded, in gW*/gb*) against target
+template <int NS>
 double backward(nt_denoiser* d, const float* target)
 {
         const long long P = d->P;
         const int P32 = (int)P;
         cudaStream_t s = d->st_use;
         int* err = d->err.as<int>();
-        const int A = d->n - 1;
+        const int A = NS - 1;
+        const int tb = pixel_threads(P);
         ck(cudaMemsetAsync(d->sums.p, 0, 2 * sizeof(double), s), "memset");
-        k_energy<<<blocks_for(P * 3), TB, 0, s>>>(P * 3, d->Y.as<float>(), target, d->sums.as<double>());
-        float* G0 = d->G.as<float>();
-        float* G1 = G0 + (size_t)P * 3;
-        k_loss_grad<<<blocks_for(P * 3), TB, 0, s>>>(P * 3, d->Y.as<float>() + (size_t)A * P * 3, target,
-                                                       d->sums.as<double>(), G0);
-        ck(cudaMemsetAsync(d->dZ.p, 0, (size_t)P * d->Op * sizeof(__nv_bfloat16), s), "memset");
-        float* gout = G0;
-        float* gin = G1;
+        k_energy<<<blocks_for(P, TB), TB, 0, s>>>((unsigned)P, image(d, 0), target, d->sums.as<double>());
+        float4* gout = d->G;
+        float4* gin = gout + P;
+        k_loss_grad<<<blocks_for(P, TB), TB, 0, s>>>((unsigned)P, image(d, A), target, d->sums.as<double>(), gout);
         for (int a = A - 1; a >= 0; --a)
         {
                 if (a > 0)
                 {
-                        ck(cudaMemsetAsync(gin, 0, (size_t)P * 3 * sizeof(float), s), "memset");
+                        ck(cudaMemsetAsync(gin, 0, (size_t)P * sizeof(float4), s), "memset");
                 }
-                k_filter_bwd<<<blocks_for(P), TB, 0, s>>>(P, d->st, a, d->base.as<float>(), d->Z.as<float>(), d->Op,
-                                                            d->Y.as<float>() + (size_t)a * P * 3, gout, a > 0 ? gin : nullptr,
-                                                            d->dZ.as<__nv_bfloat16>());
+                k_filter_bwd<NS><<<blocks_for(P, tb), tb, 0, s>>>(d->st, a, d->base, d->Z, image(d, a),
+                                                                  gout, a > 0 ? gin : nullptr, d->Op, d->dZ);
                 std::swap(gout, gin);
         }
         ck(cudaGetLastError(), "filter backward");
         // backward data products
-        ck(gemm(LoadRows{d->dZ.as<__nv_bfloat16>(), d->Op}, LoadCols{d->W3.as<__nv_bfloat16>(), HID},
-                EpiMaskBF16{d->H2.as<__nv_bfloat16>(), d->dH2.as<__nv_bfloat16>(), HID}, P32, HID, d->Op, 0, err, s),
+        ck(gemm(LoadRows{d->dZ, d->Op}, LoadCols{d->W3.as<__nv_bfloat16>(), HID},
+                EpiMaskBF16{d->H2, d->dH2, HID}, P32, HID, d->Op, 0, err, s),
            "gemm dH2");
-        ck(gemm(LoadRows{d->dH2.as<__nv_bfloat16>(), HID}, LoadCols{d->W2.as<__nv_bfloat16>(), HID},
-                EpiMaskBF16{d->H1.as<__nv_bfloat16>(), d->dH1.as<__nv_bfloat16>(), HID}, P32, HID, HID, 0, err, s),
+        ck(gemm(LoadRows{d->dH2, HID}, LoadCols{d->W2.as<__nv_bfloat16>(), HID},
+                EpiMaskBF16{d->H1, d->dH1, HID}, P32, HID, HID, 0, err, s),
            "gemm dH1");
         // weight gradients: reductions over pixels, split across CTAs, about four per SM (the products
         // are skinny and HBM-bound, so their copies need the CTAs in flight)
@@ -1222,21 +1591,22 @@ double backward(nt_denoiser* d, const float* target)
         int dev = 0, sms = 148;
         ck(cudaGetDevice(&dev), "device");
         ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
+        // at least 256 rows each: every CTA adds its whole matrix to the sum with atomics
         const long long ctas = 4LL * std::max(1, sms);
-        const int kpc = (int)std::max<long long>(GK, ((long long)P32 + ctas - 1) / ctas);
-        ck(gemm(LoadCols{d->dZ.as<__nv_bfloat16>(), d->Op}, LoadCols{d->H2.as<__nv_bfloat16>(), HID},
+        const int kpc = (int)std::max<long long>(4 * GK, ((long long)P32 + ctas - 1) / ctas);
+        ck(gemm(LoadCols{d->dZ, d->Op}, LoadCols{d->H2, HID},
                 EpiAtomicF32{d->gW3, HID, HID}, d->Op, HID, P32, kpc, err, s),
            "gemm dW3");
-        ck(gemm(LoadCols{d->dH2.as<__nv_bfloat16>(), HID}, LoadCols{d->H1.as<__nv_bfloat16>(), HID},
+        ck(gemm(LoadCols{d->dH2, HID}, LoadCols{d->H1, HID},
                 EpiAtomicF32{d->gW2, HID, HID}, HID, HID, P32, kpc, err, s),
            "gemm dW2");
-        ck(gemm(LoadCols{d->dH1.as<__nv_bfloat16>(), HID}, LoadCols{d->X.as<__nv_bfloat16>(), d->Fp},
+        ck(gemm(LoadCols{d->dH1, HID}, LoadCols{d->X, d->Fp},
                 EpiAtomicF32{d->gW1, d->Fp, d->Fp}, HID, d->Fp, P32, kpc, err, s),
            "gemm dW1");
-        const unsigned cb = (unsigned)std::min<long long>((P + 3) / 4, 1024);
-        k_colsum<<<cb, TB, 0, s>>>(P, d->Op, d->Op, d->dZ.as<__nv_bfloat16>(), d->gb3);
-        k_colsum<<<cb, TB, 0, s>>>(P, HID, HID, d->dH2.as<__nv_bfloat16>(), d->gb2);
-        k_colsum<<<cb, TB, 0, s>>>(P, HID, HID, d->dH1.as<__nv_bfloat16>(), d->gb1);
+        const ColSums cs{{d->dZ, d->dH2, d->dH1},
+                         {d->gb3, d->gb2, d->gb1},
+                         {d->Op, HID, HID}};
+        k_colsum<<<dim3((unsigned)std::min<long long>((P + 127) / 128, 256), 3), TB, 0, s>>>(P, cs);
         k_unpack<<<64, TB, 0, s>>>(d->F, d->Fp, d->O, d->gW1, d->gb1, d->gW2,
                                    d->gb2, d->gW3, d->gb3, d->g.as<float>());
         ck(cudaGetLastError(), "gradients");
@@ -1244,6 +1614,29 @@ double backward(nt_denoiser* d, const float* target)
         ck(cudaMemcpyAsync(sums, d->sums.p, sizeof(sums), cudaMemcpyDeviceToHost, s), "loss");
         check_err(d);
         return sums[1];
+}
+}
+
+namespace
+{
+// calls f with the denoiser's dimension as a compile-time constant
+template <typename F>
+void by_dimension(int n, F&& f)
+{
+        switch (n)
+        {
+        case 3:
+                f(std::integral_constant<int, 3>());
+                break;
+        case 4:
+                f(std::integral_constant<int, 4>());
+                break;
+        case 5:
+                f(std::integral_constant<int, 5>());
+                break;
+        default:
+                f(std::integral_constant<int, 6>());
+        }
 }
 }
 
@@ -1398,37 +1791,33 @@ int nt_denoiser_set_input(nt_denoiser* d, const int32_t* screen, int samples_per
                                 throw DError{NT_EINVAL, "screen sizes must be positive"};
                         }
                         st.size[a] = screen[a];
-                        st.stride[a] = P;
-                        P *= screen[a];
+                        st.stride[a] = (unsigned)std::min<long long>(P, 1LL << 31);
+                        P = P > (1LL << 30) ? P : P * screen[a];
                 }
                 if (P > (1LL << 30))
                 {
                         throw DError{NT_EINVAL, "too many pixels for the denoiser"};
                 }
                 st.nf = d->nf;
-                st.stencil_features = d->F - 1;
                 st.features = d->F;
+                st.pixels = (unsigned)P;
                 st.noise_level = (float)(1.0 / std::sqrt((double)samples_per_pixel));
                 d->st = st;
                 d->P = P;
                 d->st_use = stream ? (cudaStream_t)stream : d->own;
-                d->base.ensure(sizeof(float) * (size_t)P * BASE_STRIDE);
-                d->X.ensure(sizeof(__nv_bfloat16) * (size_t)P * d->Fp);
-                d->H1.ensure(sizeof(__nv_bfloat16) * (size_t)P * HID);
-                d->H2.ensure(sizeof(__nv_bfloat16) * (size_t)P * HID);
-                d->dH1.ensure(sizeof(__nv_bfloat16) * (size_t)P * HID);
-                d->dH2.ensure(sizeof(__nv_bfloat16) * (size_t)P * HID);
-                d->Z.ensure(sizeof(float) * (size_t)P * d->Op);
-                d->dZ.ensure(sizeof(__nv_bfloat16) * (size_t)P * d->Op);
-                d->Y.ensure(sizeof(float) * (size_t)P * 3 * d->n);
-                d->G.ensure(sizeof(float) * (size_t)P * 3 * 2);
-                k_base_features<<<blocks_for(P), TB, 0, d->st_use>>>(P, st, d_mean, d_var, d_normal, d_depth,
-                                                                      d->base.as<float>());
-                k_features<<<blocks_for(P * (d->Fp / 8)), TB, 0, d->st_use>>>(P, st, d->Fp, d->base.as<float>(),
-                                                                              d->X.as<__nv_bfloat16>());
+                d->features = false;
+                d->X = nullptr;  // forward() carves the training workspace for this image
+                const size_t bb = sizeof(float4) * (size_t)P * BASE_PLANES, yb = sizeof(float4) * (size_t)P * (d->n - 1);
+                d->infer_ws.ensure(bb + yb + sizeof(float) * (size_t)P * d->O);
+                d->base = d->infer_ws.as<float4>();
+                d->Y = d->base + (size_t)P * BASE_PLANES;
+                d->Z = (float*)(d->Y + (size_t)P * (d->n - 1));
+                const int tb = pixel_threads(P);
+                by_dimension(d->n, [&](auto ns) {
+                        k_base_features<ns><<<blocks_for(P, tb), tb, 0, d->st_use>>>(st, d_mean, d_var, d_normal, d_depth,
+                                                                                     d->base);
+                });
                 ck(cudaGetLastError(), "features");
-                ck(cudaMemcpyAsync(d->Y.p, d_mean, sizeof(float) * (size_t)P * 3, cudaMemcpyDeviceToDevice, d->st_use),
-                   "copy");
         });
 }
 
@@ -1439,10 +1828,7 @@ int nt_denoiser_apply(nt_denoiser* d, float* d_out)
                 {
                         throw DError{NT_EINVAL, "null argument"};
                 }
-                forward(d);
-                ck(cudaMemcpyAsync(d_out, d->Y.as<float>() + (size_t)(d->n - 1) * d->P * 3, sizeof(float) * (size_t)d->P * 3,
-                                   cudaMemcpyDeviceToDevice, d->st_use),
-                   "copy");
+                by_dimension(d->n, [&](auto ns) { infer<ns>(d, d_out); });
                 check_err(d);
         });
 }
@@ -1454,8 +1840,11 @@ int nt_denoiser_gradient(nt_denoiser* d, const float* d_target, float* grad, dou
                 {
                         throw DError{NT_EINVAL, "null argument"};
                 }
-                forward(d);
-                const double l = backward(d, d_target);
+                double l = 0;
+                by_dimension(d->n, [&](auto ns) {
+                        forward<ns>(d);
+                        l = backward<ns>(d, d_target);
+                });
                 if (grad)
                 {
                         ck(cudaMemcpyAsync(grad, d->g.p, sizeof(float) * d->nparams, cudaMemcpyDeviceToHost, d->st_use),
@@ -1476,8 +1865,11 @@ int nt_denoiser_train_step(nt_denoiser* d, const float* d_target, float lr, doub
                 {
                         throw DError{NT_EINVAL, "bad argument"};
                 }
-                forward(d);
-                const double l = backward(d, d_target);
+                double l = 0;
+                by_dimension(d->n, [&](auto ns) {
+                        forward<ns>(d);
+                        l = backward<ns>(d, d_target);
+                });
                 ++d->adam_t;
                 const float c1 = 1.0f - std::pow(0.9f, (float)d->adam_t);
                 const float c2 = 1.0f - std::pow(0.999f, (float)d->adam_t);
