@@ -691,16 +691,42 @@ NT_HD bool lp_feasible(const std::array<Vec<NS, T>, M>& a_in, const std::array<T
         return false;
 }
 
-// shape_intersection(box, simplex, 10 epsilons) (src/painter/space/shape_intersection.h:343-385)
+enum OverlapResult : int
+{
+        OVERLAP_NO = 0,
+        OVERLAP_YES = 1,
+        OVERLAP_LP = 2  // the linear program decides (box_simplex_lp)
+};
+
+// The constraints of a box: x_i <= d1_i and -x_i <= d2_i (a . x + b >= 0).
 template <int N, typename T>
-NT_HD bool box_simplex_overlap(const Box<N, T>& box, const SimplexShape<N, T>& s)
+NT_HD std::array<Constraint<N, T>, 2 * N> box_constraints(const Box<N, T>& box)
+{
+        std::array<Constraint<N, T>, 2 * N> bc;
+        for (int i = 0; i < N; ++i)
+        {
+                for (int k = 0; k < N; ++k)
+                {
+                        bc[2 * i].a[k] = (k == i) ? T(-1) : T(0);
+                        bc[2 * i + 1].a[k] = (k == i) ? T(1) : T(0);
+                }
+                bc[2 * i].b = box.d1[i];
+                bc[2 * i + 1].b = box.d2[i];
+        }
+        return bc;
+}
+
+// shape_intersection(box, simplex, 10 epsilons) (src/painter/space/shape_intersection.h:343-385) up to
+// the linear program: vertices inside the box, segments (n <= 3), separating planes.
+template <int N, typename T>
+NT_HD OverlapResult box_simplex_quick(const Box<N, T>& box, const SimplexShape<N, T>& s)
 {
         constexpr int VC = 1 << N;
         for (int i = 0; i < N; ++i)
         {
                 if (box.inside(s.v[i]))
                 {
-                        return true;
+                        return OVERLAP_YES;
                 }
         }
         if constexpr (N <= 3)
@@ -728,7 +754,7 @@ NT_HD bool box_simplex_overlap(const Box<N, T>& box, const SimplexShape<N, T>& s
                                 e[i] = box.size[i];
                                 if (seg_hits_simplex(v, e))
                                 {
-                                        return true;
+                                        return OVERLAP_YES;
                                 }
                         }
                 }
@@ -743,26 +769,16 @@ NT_HD bool box_simplex_overlap(const Box<N, T>& box, const SimplexShape<N, T>& s
                                 }
                                 if (seg_hits_box(s.v[i], d))
                                 {
-                                        return true;
+                                        return OVERLAP_YES;
                                 }
                         }
                 }
-                return false;
+                return OVERLAP_NO;
         }
         else
         {
                 // shapes_not_intersect_by_planes
-                std::array<Constraint<N, T>, 2 * N> bc;
-                for (int i = 0; i < N; ++i)
-                {
-                        for (int k = 0; k < N; ++k)
-                        {
-                                bc[2 * i].a[k] = (k == i) ? T(-1) : T(0);
-                                bc[2 * i + 1].a[k] = (k == i) ? T(1) : T(0);
-                        }
-                        bc[2 * i].b = box.d1[i];
-                        bc[2 * i + 1].b = box.d2[i];
-                }
+                const std::array<Constraint<N, T>, 2 * N> bc = box_constraints<N, T>(box);
                 for (const auto& c : bc)
                 {
                         bool all_negative = true;
@@ -776,7 +792,7 @@ NT_HD bool box_simplex_overlap(const Box<N, T>& box, const SimplexShape<N, T>& s
                         }
                         if (all_negative)
                         {
-                                return false;
+                                return OVERLAP_NO;
                         }
                 }
                 std::array<Vec<N, T>, VC> bv;
@@ -797,7 +813,7 @@ NT_HD bool box_simplex_overlap(const Box<N, T>& box, const SimplexShape<N, T>& s
                         }
                         if (all_negative)
                         {
-                                return false;
+                                return OVERLAP_NO;
                         }
                 }
                 {
@@ -816,48 +832,69 @@ NT_HD bool box_simplex_overlap(const Box<N, T>& box, const SimplexShape<N, T>& s
                         }
                         if (same)
                         {
-                                return false;
+                                return OVERLAP_NO;
                         }
                 }
-                // shapes_intersect_by_spaces
-                Vec<N, T> mn;
-                T max_value = 0;
-                for (int k = 0; k < N; ++k)
-                {
-                        mn[k] = smin(box.org[k], s.min[k]);
-                }
-                for (int k = 0; k < N; ++k)
-                {
-                        T d = smax(box.org[k] + box.size[k], s.max[k]) - mn[k];
-                        max_value = (k == 0) ? d : smax(max_value, d);
-                }
-                const T distance = max_value * (T(10) * std::numeric_limits<T>::epsilon());
-                constexpr int M = 3 * N + 2;
-                std::array<Vec<N, T>, M> a;
-                std::array<T, M> b;
-                int i = 0;
-                for (const auto& c : bc)
-                {
-                        a[i] = c.a;
-                        b[i] = dot<N, T>(c.a, mn) + c.b;
-                        ++i;
-                }
-                for (const auto& c : s.c)
-                {
-                        a[i] = c.a;
-                        b[i] = dot<N, T>(c.a, mn) + c.b;
-                        ++i;
-                }
-                T b_v = dot<N, T>(s.c_eq.a, mn) + s.c_eq.b;
-                a[i] = s.c_eq.a;
-                b[i] = b_v + distance;
-                ++i;
-                for (int k = 0; k < N; ++k)
-                {
-                        a[i][k] = -s.c_eq.a[k];
-                }
-                b[i] = -b_v + distance;
-                return lp_feasible<N, T, M>(a, b);
+                return OVERLAP_LP;
         }
+}
+
+// shapes_intersect_by_spaces: the feasibility of the box's and the simplex's constraints together (n >= 4)
+template <int N, typename T>
+NT_HD bool box_simplex_lp(const Box<N, T>& box, const SimplexShape<N, T>& s)
+{
+        const std::array<Constraint<N, T>, 2 * N> bc = box_constraints<N, T>(box);
+        Vec<N, T> mn;
+        T max_value = 0;
+        for (int k = 0; k < N; ++k)
+        {
+                mn[k] = smin(box.org[k], s.min[k]);
+        }
+        for (int k = 0; k < N; ++k)
+        {
+                T d = smax(box.org[k] + box.size[k], s.max[k]) - mn[k];
+                max_value = (k == 0) ? d : smax(max_value, d);
+        }
+        const T distance = max_value * (T(10) * std::numeric_limits<T>::epsilon());
+        constexpr int M = 3 * N + 2;
+        std::array<Vec<N, T>, M> a;
+        std::array<T, M> b;
+        int i = 0;
+        for (const auto& c : bc)
+        {
+                a[i] = c.a;
+                b[i] = dot<N, T>(c.a, mn) + c.b;
+                ++i;
+        }
+        for (const auto& c : s.c)
+        {
+                a[i] = c.a;
+                b[i] = dot<N, T>(c.a, mn) + c.b;
+                ++i;
+        }
+        T b_v = dot<N, T>(s.c_eq.a, mn) + s.c_eq.b;
+        a[i] = s.c_eq.a;
+        b[i] = b_v + distance;
+        ++i;
+        for (int k = 0; k < N; ++k)
+        {
+                a[i][k] = -s.c_eq.a[k];
+        }
+        b[i] = -b_v + distance;
+        return lp_feasible<N, T, M>(a, b);
+}
+
+template <int N, typename T>
+NT_HD bool box_simplex_overlap(const Box<N, T>& box, const SimplexShape<N, T>& s)
+{
+        const OverlapResult r = box_simplex_quick<N, T>(box, s);
+        if constexpr (N > 3)
+        {
+                if (r == OVERLAP_LP)
+                {
+                        return box_simplex_lp<N, T>(box, s);
+                }
+        }
+        return r == OVERLAP_YES;
 }
 }

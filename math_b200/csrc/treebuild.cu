@@ -2,11 +2,11 @@
 //
 // Level by level, as the host build: the boxes of a level that hold more than min_objects facets (and
 // are above the depth limit) split into 2^N children with contiguous node numbers in parent order.
-// For every child, one block tests the parent's facets against the child box (box_simplex_overlap,
-// the host's code compiled for the device) and records the outcomes as a bit mask (warp ballots) and
-// a count; after a prefix sum of the counts on the host, one warp per child writes the facets that
-// overlap, in the parent's list order.  Leaves keep their level's list; the leaf index array is their
-// lists in node order (breadth-first numbering makes level order node order).
+// The parent's facets are tested against each child box (box_simplex_overlap's parts, the host's code
+// compiled for the device) and the outcomes recorded as a bit mask and a count per child; after a prefix
+// sum of the counts on the host, one warp per child writes the facets that overlap, in the parent's list
+// order.  Leaves keep their level's list; the leaf index array is their lists in node order (breadth-first
+// numbering makes level order node order).
 #include "treebuild.h"
 
 #include <algorithm>
@@ -16,7 +16,7 @@ namespace ntrace
 {
 namespace
 {
-constexpr int TB = 256;
+constexpr int TB = 128;
 
 template <int N>
 struct ChildDesc
@@ -27,51 +27,110 @@ struct ChildDesc
         long long word_off;   // this child's segment of the bit masks
 };
 
+// word_child[w] = the child whose bit mask holds word w (one warp per child)
+template <int N>
+__global__ void __launch_bounds__(TB) k_word_child(const ChildDesc<N>* __restrict__ kids, long long nkids,
+                                                   int* __restrict__ word_child)
+{
+        const int lane = threadIdx.x & 31;
+        const long long warps = (long long)gridDim.x * (TB / 32);
+        for (long long c = (long long)blockIdx.x * (TB / 32) + (threadIdx.x >> 5); c < nkids; c += warps)
+        {
+                const long long off = kids[c].word_off;
+                const long long words = (kids[c].list_cnt + 31) >> 5;
+                for (long long w = lane; w < words; w += 32)
+                {
+                        word_child[off + w] = (int)c;
+                }
+        }
+}
+
+// The overlap of every (child box, facet of its parent's list) pair of a level: a warp takes one word of
+// the bit masks at a time, 32 facets of one child.  Most pairs are settled by the quick tests; the others
+// wait in shared memory until the warp has 32 of them, so that the linear program, by far the longest
+// part, runs on full warps instead of on the few lanes of a word that need it, and the work is spread
+// over the words of the level, not its children (16 of them, with the whole mesh in each, at the top; a
+// million with a dozen facets at the bottom).  The tests and their order are the host's
+// (box_simplex_overlap).
 template <int N>
 __global__ void __launch_bounds__(TB) k_overlap(const SimplexShape<N, float>* __restrict__ shapes,
                                                 const int* __restrict__ list_cur, const ChildDesc<N>* __restrict__ kids,
-                                                long long nkids, Vec<N, float> half, unsigned* __restrict__ bits,
-                                                unsigned* __restrict__ counts, unsigned long long* tests)
+                                                const int* __restrict__ word_child, long long nwords, Vec<N, float> half,
+                                                unsigned* __restrict__ bits, unsigned* __restrict__ counts)
 {
-        __shared__ unsigned s_count;
-        const int lane = threadIdx.x & 31;
-        const int warp = threadIdx.x >> 5;
-        for (long long c = blockIdx.x; c < nkids; c += gridDim.x)
+        struct Pending
         {
+                long long word;
+                int child;
+                int facet;
+                int lane;
+        };
+        __shared__ Pending s_pending[TB / 32][64];
+        Pending* const pending = s_pending[threadIdx.x >> 5];
+        const unsigned full = 0xffffffffu;
+        const int lane = threadIdx.x & 31;
+        const unsigned lt = (1u << lane) - 1;
+        const long long warps = (long long)gridDim.x * (TB / 32);
+        int waiting = 0;
+        auto settle = [&](int first, int count) {
+                __syncwarp();
+                if (lane < count)
+                {
+                        const Pending p = pending[first + lane];
+                        const Box<N, float> box = Box<N, float>::make(kids[p.child].org, half);
+                        bool hit = true;
+                        if constexpr (N > 3)
+                        {
+                                hit = box_simplex_lp<N, float>(box, shapes[p.facet]);
+                        }
+                        if (hit)
+                        {
+                                atomicOr(bits + p.word, 1u << p.lane);
+                                atomicAdd(counts + p.child, 1u);
+                        }
+                }
+                __syncwarp();
+        };
+        for (long long w = (long long)blockIdx.x * (TB / 32) + (threadIdx.x >> 5); w < nwords; w += warps)
+        {
+                const int c = word_child[w];
                 const ChildDesc<N> d = kids[c];
-                const Box<N, float> box = Box<N, float>::make(d.org, half);
-                if (threadIdx.x == 0)
+                const long long j = (w - d.word_off) * 32 + lane;
+                OverlapResult r = OVERLAP_NO;
+                int f = 0;
+                if (j < d.list_cnt)
                 {
-                        s_count = 0;
+                        f = list_cur[d.list_off + j];
+                        r = box_simplex_quick<N, float>(Box<N, float>::make(d.org, half), shapes[f]);
                 }
-                __syncthreads();
-                unsigned mine = 0;
-                for (long long j0 = 0; j0 < d.list_cnt; j0 += TB)
-                {
-                        const long long j = j0 + threadIdx.x;
-                        bool hit = false;
-                        if (j < d.list_cnt)
-                        {
-                                hit = box_simplex_overlap<N, float>(box, shapes[list_cur[d.list_off + j]]);
-                        }
-                        const unsigned b = __ballot_sync(0xffffffffu, hit);
-                        if (lane == 0 && j0 + warp * 32 < d.list_cnt)
-                        {
-                                bits[d.word_off + (j0 >> 5) + warp] = b;
-                                mine += __popc(b);
-                        }
-                }
+                const unsigned yes = __ballot_sync(full, r == OVERLAP_YES);
+                const unsigned open = __ballot_sync(full, r == OVERLAP_LP);
                 if (lane == 0)
                 {
-                        atomicAdd(&s_count, mine);
+                        bits[w] = yes;
+                        if (yes)
+                        {
+                                atomicAdd(counts + c, (unsigned)__popc(yes));
+                        }
                 }
-                __syncthreads();
-                if (threadIdx.x == 0)
+                if (r == OVERLAP_LP)
                 {
-                        counts[c] = s_count;
-                        atomicAdd(tests, (unsigned long long)d.list_cnt);
+                        Pending& p = pending[waiting + __popc(open & lt)];
+                        p.word = w;
+                        p.child = c;
+                        p.facet = f;
+                        p.lane = lane;
                 }
-                __syncthreads();
+                waiting += __popc(open);
+                if (waiting >= 32)
+                {
+                        settle(waiting - 32, 32);
+                        waiting -= 32;
+                }
+        }
+        if (waiting > 0)
+        {
+                settle(0, waiting);
         }
 }
 
@@ -111,14 +170,24 @@ struct Dev
                         cudaFree(p);
                 }
         }
-        cudaError_t alloc(size_t bytes)
+        size_t bytes = 0;
+        // room for at least n bytes; the contents are not kept when it grows
+        cudaError_t alloc(size_t n)
         {
+                if (n <= bytes)
+                {
+                        return cudaSuccess;
+                }
                 if (p)
                 {
                         cudaFree(p);
                         p = nullptr;
+                        bytes = 0;
                 }
-                return cudaMalloc(&p, std::max<size_t>(bytes, 16));
+                n = std::max<size_t>(n, 16);
+                const cudaError_t e = cudaMalloc(&p, n);
+                bytes = e == cudaSuccess ? n : 0;
+                return e;
         }
 };
 
@@ -142,13 +211,13 @@ void build_tree_gpu(const std::vector<SimplexShape<N, float>>& shapes, const Vec
 {
         const long long nf = (long long)shapes.size();
         constexpr int C = 1 << N;
-        Dev d_shapes, d_tests;
+        Dev d_shapes;
+        Dev d_kids, d_bits, d_counts, d_off, d_child;  // a level's work memory, kept for the next one
         TB_CHECK(d_shapes.alloc(sizeof(SimplexShape<N, float>) * (size_t)nf), "cudaMalloc");
         TB_CHECK(cudaMemcpyAsync(d_shapes.p, shapes.data(), sizeof(SimplexShape<N, float>) * (size_t)nf,
                                  cudaMemcpyHostToDevice, st),
                  "upload");
-        TB_CHECK(d_tests.alloc(sizeof(unsigned long long)), "cudaMalloc");
-        TB_CHECK(cudaMemsetAsync(d_tests.p, 0, sizeof(unsigned long long), st), "memset");
+        unsigned long long tests = 0;
 
         // one list buffer per level (leaves keep pointing into theirs)
         std::vector<std::unique_ptr<Dev>> lists;
@@ -229,21 +298,26 @@ void build_tree_gpu(const std::vector<SimplexShape<N, float>>& shapes, const Vec
                                 d.list_cnt = parent.cnt;
                                 d.word_off = words;
                                 words += (parent.cnt + 31) / 32;
+                                tests += (unsigned long long)parent.cnt;
                         }
                 }
-                Dev d_kids, d_bits, d_counts, d_off;
                 TB_CHECK(d_kids.alloc(sizeof(ChildDesc<N>) * (size_t)nkids), "cudaMalloc");
                 TB_CHECK(d_bits.alloc(sizeof(unsigned) * (size_t)words), "cudaMalloc");
                 TB_CHECK(d_counts.alloc(sizeof(unsigned) * (size_t)nkids), "cudaMalloc");
                 TB_CHECK(cudaMemcpyAsync(d_kids.p, kids.data(), sizeof(ChildDesc<N>) * (size_t)nkids, cudaMemcpyHostToDevice,
                                          st),
                          "upload");
-                const unsigned grid = (unsigned)std::min<long long>(nkids, 148LL * 64);
+                TB_CHECK(d_child.alloc(sizeof(int) * (size_t)words), "cudaMalloc");
+                TB_CHECK(cudaMemsetAsync(d_counts.p, 0, sizeof(unsigned) * (size_t)nkids, st), "memset");
+                const unsigned cgrid = (unsigned)std::min<long long>((nkids + TB / 32 - 1) / (TB / 32), 148LL * 64);
+                k_word_child<N><<<cgrid, TB, 0, st>>>(static_cast<const ChildDesc<N>*>(d_kids.p), nkids,
+                                                      static_cast<int*>(d_child.p));
+                const unsigned grid = (unsigned)std::min<long long>((words + TB / 32 - 1) / (TB / 32), 148LL * 16);
                 k_overlap<N><<<grid, TB, 0, st>>>(static_cast<const SimplexShape<N, float>*>(d_shapes.p),
                                                   static_cast<const int*>(lists[level]->p),
-                                                  static_cast<const ChildDesc<N>*>(d_kids.p), nkids, half,
-                                                  static_cast<unsigned*>(d_bits.p), static_cast<unsigned*>(d_counts.p),
-                                                  static_cast<unsigned long long*>(d_tests.p));
+                                                  static_cast<const ChildDesc<N>*>(d_kids.p),
+                                                  static_cast<const int*>(d_child.p), words, half,
+                                                  static_cast<unsigned*>(d_bits.p), static_cast<unsigned*>(d_counts.p));
                 TB_CHECK(cudaGetLastError(), "overlap kernel");
                 std::vector<unsigned> counts((size_t)nkids);
                 TB_CHECK(cudaMemcpyAsync(counts.data(), d_counts.p, sizeof(unsigned) * (size_t)nkids, cudaMemcpyDeviceToHost,
@@ -284,8 +358,8 @@ void build_tree_gpu(const std::vector<SimplexShape<N, float>>& shapes, const Vec
                 }
                 cur.swap(next);
         }
-        // leaf lists in node order (levels are in node order, and so are the boxes within a level)
-        std::sort(leaves.begin(), leaves.end(), [](const LeafRef& a, const LeafRef& b) { return a.node < b.node; });
+        // leaf lists in node order, which is the order the leaves were found in: level by level, and by node
+        // within a level
         std::vector<std::vector<int>> host_lists(lists.size());
         for (size_t l = 0; l < lists.size(); ++l)
         {
@@ -297,10 +371,14 @@ void build_tree_gpu(const std::vector<SimplexShape<N, float>>& shapes, const Vec
                                  "copy");
                 }
         }
-        unsigned long long tests = 0;
-        TB_CHECK(cudaMemcpyAsync(&tests, d_tests.p, sizeof(tests), cudaMemcpyDeviceToHost, st), "copy");
         TB_CHECK(cudaStreamSynchronize(st), "sync");
         out->leaf_idx.clear();
+        size_t references = 0;
+        for (const LeafRef& lf : leaves)
+        {
+                references += (size_t)lf.cnt;
+        }
+        out->leaf_idx.reserve(std::max<size_t>(references, 1));
         for (const LeafRef& lf : leaves)
         {
                 nodes[lf.node * 2 + 0] = (int32_t)out->leaf_idx.size();
