@@ -27,12 +27,15 @@ constexpr int shade_min_blocks()
 {
         return N == 3 ? 8 : 6;
 }
-// at n = 6 the walk state is larger: one block fewer, so that 128 registers fit without spills
+// from n = 5 on the walk state is larger: one block fewer, so that 128 registers fit without spills (n = 5
+// frame: extension 3.63 -> 3.43 ms, shadow walk 5.69 -> 5.43; at n = 4 the fifth block is worth its spills,
+// 23.9 against 26.5 ms)
 template <int N>
 constexpr int walk_min_blocks()
 {
-        return (N >= 6 && WALK_MIN_BLOCKS > 1) ? WALK_MIN_BLOCKS - 1 : WALK_MIN_BLOCKS;
+        return (N >= 5 && WALK_MIN_BLOCKS > 1) ? WALK_MIN_BLOCKS - 1 : WALK_MIN_BLOCKS;
 }
+
 __device__ __forceinline__ unsigned lanemask_lt()
 {
         unsigned m;
@@ -250,13 +253,6 @@ struct ShadowView
                 return f[field * Q + i];
         }
 };
-
-__device__ __forceinline__ uint32_t fast_div(const FastDiv& f, uint32_t n, uint32_t* rest)
-{
-        const uint32_t q = (uint32_t)(((unsigned long long)n * f.m) >> f.s);
-        *rest = n - q * f.d;
-        return q;
-}
 
 // paint_pixels: stratified jittered sample -> projector ray (painter.cpp:410-448,
 // sampler.h:26-64, engine.h:86-156)
@@ -1144,7 +1140,7 @@ __global__ void k_moments_reduce(long long npix, int spp, const double* __restri
 
 // Start of a wavefront iteration (one thread): refill the queue with fresh paths up to Q and clear the
 // per-iteration counters.
-__global__ void k_iter_begin(unsigned long long* c, long long total, long long Q, int parity)
+__device__ __forceinline__ void iteration_begin(unsigned long long* c, long long total, long long Q, int parity)
 {
         const long long active = (long long)c[C_Q_ACTIVE];
         const long long next = (long long)c[C_Q_NEXT];
@@ -1167,13 +1163,22 @@ __global__ void k_iter_begin(unsigned long long* c, long long total, long long Q
         }
 }
 
+__global__ void k_iter_begin(unsigned long long* c, long long total, long long Q, int parity)
+{
+        iteration_begin(c, total, Q, parity);
+}
+
 // End of an iteration (one thread): the continuations become the queue; done once every path of the
-// pass has been generated and finished.
-__global__ void k_iter_end(unsigned long long* c, long long total)
+// pass has been generated and finished.  next_parity >= 0: the next iteration begins here too.
+__global__ void k_iter_end(unsigned long long* c, long long total, long long Q, int next_parity)
 {
         const long long survivors = (long long)c[C_ACTIVE_OUT];
         c[C_Q_ACTIVE] = (unsigned long long)survivors;
         c[C_DONE] = (survivors == 0 && (long long)c[C_Q_NEXT] >= total) ? 1ull : 0ull;
+        if (next_parity >= 0)
+        {
+                iteration_begin(c, total, Q, next_parity);
+        }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1329,7 +1334,7 @@ const LaunchSizes& Wavefront<N>::prepare()
 template <int N>
 void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, double* accum, unsigned long long* counters,
                                      long long total_paths, int parity, cudaStream_t st, KernelTimes* times,
-                                     cudaEvent_t* ev, const SideStream* side) const
+                                     cudaEvent_t* ev, const SideStream* side, bool begun, bool begin_next) const
 {
         const LaunchSizes& L = prepare();
         const long long extend_blocks = L.extend_blocks;
@@ -1357,7 +1362,10 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         HitView<N> H{hit_t, hit_obj, hit_facet};
         ShadowView<N> SQ{sq_f, sq_pix, Q * lights};
         ShadowView<N> SM{sm_f, sm_pix, Q * lights};
-        k_iter_begin<<<1, 1, 0, st>>>(counters, total_paths, Q, parity);
+        if (!begun)
+        {
+                k_iter_begin<<<1, 1, 0, st>>>(counters, total_paths, Q, parity);
+        }
         if (ev)
         {
                 cudaEventRecord(ev[0], st);
@@ -1405,8 +1413,12 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         }
         if (side)
         {
-                // the previous iteration's shadow walks read the queue that shading fills
+                // the previous iteration's shadow walks read the queues that shading fills
                 cudaStreamWaitEvent(st, side->join, 0);
+                if (smooth)
+                {
+                        cudaStreamWaitEvent(st, side->join_smooth, 0);
+                }
         }
         k_shade<N><<<shade_grid, BLOCK, 0, st>>>(S, P, A, H, B, SQ, SM, accum, counters, parity);
         if (ev)
@@ -1447,22 +1459,33 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         {
                 k_shadow<N><<<sh_grid, BLOCK, 0, sh>>>(S, SQ, accum, counters, parity);
         }
-        if (smooth)
-        {
-                k_shadow_smooth<N><<<shade_grid, BLOCK, 0, sh>>>(S, SM, accum, counters, parity);
-        }
         if (side)
         {
                 cudaEventRecord(side->join, sh);
+        }
+        if (smooth)
+        {
+                // its rays are few and walk three times in a row: beside the other shadow rays
+                cudaStream_t sm = st;
+                if (side)
+                {
+                        sm = side->smooth;
+                        cudaStreamWaitEvent(sm, side->fork, 0);
+                }
+                k_shadow_smooth<N><<<shade_grid, BLOCK, 0, sm>>>(S, SM, accum, counters, parity);
+                if (side)
+                {
+                        cudaEventRecord(side->join_smooth, sm);
+                }
         }
         if (ev)
         {
                 cudaEventRecord(ev[6], st);
         }
-        k_iter_end<<<1, 1, 0, st>>>(counters, total_paths);
+        k_iter_end<<<1, 1, 0, st>>>(counters, total_paths, Q, begin_next ? parity ^ 1 : -1);
         if (times)
         {
-                times->launches += iteration_launches(smooth, one_mesh);
+                times->launches += iteration_launches(smooth, one_mesh) - (begun ? 1 : 0);
                 times->extend_launches += 1;
                 times->shadow_launches += 1;
         }
@@ -1480,14 +1503,16 @@ void Wavefront<N>::enqueue_iterations(const DevScene<N>& S, const PassDev& P, do
         if (side)
         {
                 cudaEventRecord(side->join, st);
+                cudaEventRecord(side->join_smooth, st);
         }
         for (int k = 0; k < count; ++k)
         {
-                enqueue_iteration(S, P, accum, counters, total_paths, k & 1, st, times, nullptr, side);
+                enqueue_iteration(S, P, accum, counters, total_paths, k & 1, st, times, nullptr, side, k > 0, k + 1 < count);
         }
         if (side)
         {
                 cudaStreamWaitEvent(st, side->join, 0);
+                cudaStreamWaitEvent(st, side->join_smooth, 0);
         }
 }
 
@@ -1533,7 +1558,7 @@ cudaError_t Wavefront<N>::run(const DevScene<N>& S, PassDev P, double* accum, un
                 {
                         for (int k = 0; k < even; ++k)
                         {
-                                enqueue_iteration(S, P, accum, counters, total_paths, k & 1, st, times, ev, nullptr);
+                                enqueue_iteration(S, P, accum, counters, total_paths, k & 1, st, times, ev, nullptr, false, false);
                                 cudaEventRecord(ev[7], st);
                                 cudaEventSynchronize(ev[7]);
                                 float ms;

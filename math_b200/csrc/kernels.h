@@ -39,13 +39,15 @@ struct LaunchSizes
         long long shade_blocks = 1;
 };
 
-// A second stream for the kernels of an iteration that the next one does not wait for, and the events that
-// tie it to the pass's stream.
+// Streams for the kernels of an iteration that the next one does not wait for (the shadow walks, and the
+// smooth-normal branch's), and the events that tie them to the pass's stream.
 struct SideStream
 {
         cudaStream_t stream = nullptr;
+        cudaStream_t smooth = nullptr;
         cudaEvent_t fork = nullptr;
         cudaEvent_t join = nullptr;
+        cudaEvent_t join_smooth = nullptr;
 };
 
 // Wavefront path pool: path state A/B (double-buffered, compacted every bounce), the hit record and
@@ -94,10 +96,11 @@ struct Wavefront
         // One wavefront iteration on stream st (k_iter_begin .. k_iter_end; the queue sizes live in
         // counters, so nothing waits for the host).  parity selects which double-buffered queue is
         // current; ev (8 events, optional) are recorded around the kernel kinds; side (optional): the shadow
-        // walks' stream, joined by the next iteration's shading.  Capturable.
+        // walks' stream, joined by the next iteration's shading; begun /
+        // begin_next: the previous iteration's last kernel began this one / this one's begins the next.
         void enqueue_iteration(const DevScene<N>& S, const PassDev& P, double* accum, unsigned long long* counters,
                                long long total_paths, int parity, cudaStream_t st, KernelTimes* times,
-                               cudaEvent_t* ev, const SideStream* side) const;
+                               cudaEvent_t* ev, const SideStream* side, bool begun, bool begin_next) const;
         void enqueue_iterations(const DevScene<N>& S, const PassDev& P, double* accum, unsigned long long* counters,
                                 long long total_paths, int count, cudaStream_t st, KernelTimes* times,
                                 const SideStream* side) const;

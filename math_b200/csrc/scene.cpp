@@ -371,11 +371,14 @@ struct nt_scene
                 {
                         cudaFreeHost(host_counters);
                 }
-                if (side.stream)
+                for (cudaStream_t t : {side.stream, side.smooth})
                 {
-                        cudaStreamDestroy(side.stream);
+                        if (t)
+                        {
+                                cudaStreamDestroy(t);
+                        }
                 }
-                for (cudaEvent_t e : {side.fork, side.join})
+                for (cudaEvent_t e : {side.fork, side.join, side.join_smooth})
                 {
                         if (e)
                         {
@@ -1072,11 +1075,13 @@ void build_scene(nt_scene* s, unsigned threads, bool host_only, bool tree_on_gpu
         {
                 check_cuda(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "cudaStreamCreate");
         }
-        if (!host_only && !s->side.join)
+        if (!host_only && !s->side.join_smooth)
         {
                 check_cuda(cudaStreamCreateWithFlags(&s->side.stream, cudaStreamNonBlocking), "cudaStreamCreate");
+                check_cuda(cudaStreamCreateWithFlags(&s->side.smooth, cudaStreamNonBlocking), "cudaStreamCreate");
                 check_cuda(cudaEventCreateWithFlags(&s->side.fork, cudaEventDisableTiming), "cudaEventCreate");
                 check_cuda(cudaEventCreateWithFlags(&s->side.join, cudaEventDisableTiming), "cudaEventCreate");
+                check_cuda(cudaEventCreateWithFlags(&s->side.join_smooth, cudaEventDisableTiming), "cudaEventCreate");
         }
         for (auto& m : s->meshes)
         {
@@ -1410,7 +1415,18 @@ struct PassJobN final : PassJob
         cudaError_t run(const nt_render_opts& o) override
         {
                 return W.run(S, P, accum, s->counters.as<unsigned long long>(), s->host_counters, total, s->stream, &times,
-                             o.timing != 0, o.stop, o.graph_iterations > 0 ? o.graph_iterations : 4, &s->side);
+                             o.timing != 0, o.stop, iterations(o), &s->side);
+        }
+        // Iterations between host checks.  A pass whose pool holds all its paths ends with its deepest
+        // bounce, after max_depth + 1 iterations at most: up to 8 they are enqueued at once, without the
+        // check after four and the empty iterations that fill up the second four.
+        int iterations(const nt_render_opts& o) const
+        {
+                if (o.graph_iterations > 0)
+                {
+                        return o.graph_iterations;
+                }
+                return W.Q >= total && S.max_depth < 8 ? std::max(2, S.max_depth + 1) : 4;
         }
 };
 
@@ -1451,23 +1467,6 @@ struct PassTarget
 long long pass_first_sample(const nt_scene* s, const nt_render_opts& o)
 {
         return o.sample_offset > 0 ? (long long)o.sample_offset : s->samples_done;
-}
-
-FastDiv fast_divisor(long long d)
-{
-        FastDiv f{1, 0x80000001u, 31};
-        if (d > 0 && d < (1ll << 31))
-        {
-                int l = 0;
-                while ((1ll << l) < d)
-                {
-                        ++l;
-                }
-                f.d = (uint32_t)d;
-                f.s = (uint32_t)(31 + l);
-                f.m = (uint32_t)((1ull << (31 + l)) / (unsigned long long)d + 1);
-        }
-        return f;
 }
 
 // The constants ray generation divides by (raygen_one).

@@ -166,6 +166,31 @@ NT_HD inline unsigned child_bits(unsigned code, int s)
         return c;
 }
 
+// The constants of a division by d (FastDiv), 1 <= d < 2^31; other d give those of 1.
+inline FastDiv fast_divisor(long long d)
+{
+        FastDiv f{1, 0x80000001u, 31};
+        if (d > 0 && d < (1ll << 31))
+        {
+                int l = 0;
+                while ((1ll << l) < d)
+                {
+                        ++l;
+                }
+                f.d = (uint32_t)d;
+                f.s = (uint32_t)(31 + l);
+                f.m = (uint32_t)((1ull << (31 + l)) / (unsigned long long)d + 1);
+        }
+        return f;
+}
+
+NT_HD inline uint32_t fast_div(const FastDiv& f, uint32_t n, uint32_t* rest)
+{
+        const uint32_t q = (uint32_t)(((unsigned long long)n * f.m) >> f.s);
+        *rest = n - q * f.d;
+        return q;
+}
+
 // The exit from a leaf: the distance to the far face (ParallelotopeOrtho::intersect_impl's second
 // distance), the point there, and the face it lies on (the nearest face, parallelotope_ortho.h:337-362).
 template <int N>

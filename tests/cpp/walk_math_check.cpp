@@ -268,8 +268,36 @@ bool check(int trees, int points)
 }
 }
 
+namespace
+{
+// divisors small, large and beside powers of two; dividends at multiples and at the ends of the range
+bool check_division(int rounds)
+{
+        std::mt19937_64 rng(3);
+        for (int it = 0; it < rounds; ++it)
+        {
+                const int bits = (int)(rng() % 31);
+                long long d = it % 3 == 0 ? 1 + (long long)(rng() % 2000) : (1ll << bits) + (long long)(rng() % 3) - 1;
+                d = std::min(std::max(d, 1ll), (1ll << 31) - 1);
+                const FastDiv f = fast_divisor(d);
+                const long long top = (1ll << 31) - 1;
+                for (long long n : {0ll, 1ll, d - 1, d, d + 1, top, top - 1, top / d * d, top / d * d - 1, (long long)(rng() >> 33)})
+                {
+                        n = std::min(std::max(n, 0ll), top);
+                        uint32_t rest;
+                        if (fast_div(f, (uint32_t)n, &rest) != n / d || rest != n % d)
+                        {
+                                std::printf("%lld / %lld by multiplication differs\n", n, d);
+                                return false;
+                        }
+                }
+        }
+        return true;
+}
+}
+
 int main(int argc, char** argv)
 {
         const int points = argc > 1 ? std::atoi(argv[1]) : 2000;
-        return check<3>(60, points) && check<4>(60, points) && check<5>(60, points) && check<6>(60, points) ? 0 : 1;
+        return check_division(50 * points) && check<3>(60, points) && check<4>(60, points) && check<5>(60, points) && check<6>(60, points) ? 0 : 1;
 }

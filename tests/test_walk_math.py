@@ -1,6 +1,7 @@
 """The walk's shared arithmetic (math_b200/csrc/walk_math.hpp) against the routines it stands in for, on
-the host: the finest-cell index of a point against the descent, and the exit by approximate quotients
-against the exact slabs, for points on, beside and between box boundaries.  Where the fast rule says it
+the host: the finest-cell index of a point against the descent, the exit by approximate quotients
+against the exact slabs, for points on, beside and between box boundaries, and the division of path and
+pixel numbers by multiplication against the integer division.  Where the fast rule says it
 can decide, the result must be the exact one's."""
 
 import os
