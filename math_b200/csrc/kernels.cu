@@ -258,7 +258,7 @@ struct ShadowView
 // sampler.h:26-64, engine.h:86-156)
 template <int N>
 __device__ __forceinline__ void raygen_one(const DevScene<N>& S, const PassDev& P, const PathView<N>& A, long long g,
-                                           long long slot)
+                                           long long slot, Ray<N>& ray)
 {
         long long entry, pixel;
         int s;
@@ -315,7 +315,6 @@ __device__ __forceinline__ void raygen_one(const DevScene<N>& S, const PassDev& 
                 float sample_j = offset + u[j] * P.recip_k;
                 point[j] = (float)px[j] + sample_j;
         }
-        Ray<N> ray;
         projector_ray<N>(S.proj, point, ray);
 #pragma unroll
         for (int k = 0; k < N; ++k)
@@ -323,26 +322,84 @@ __device__ __forceinline__ void raygen_one(const DevScene<N>& S, const PassDev& 
                 A.at(k, slot) = ray.org[k];
                 A.at(N + k, slot) = ray.dir[k];
         }
-        A.at(2 * N + 0, slot) = 1.0f;
-        A.at(2 * N + 1, slot) = 1.0f;
-        A.at(2 * N + 2, slot) = 1.0f;
-        A.at(2 * N + 3, slot) = 1.0f;
+        // throughput 1, colour level 1 and bounce level 0 are not stored: a path is fresh while its slot
+        // is at or past C_Q_BASE
         A.pix[slot] = P.moments ? (uint32_t)g : (uint32_t)entry;
         A.smp[slot] = (uint32_t)sample;
-        A.level[slot] = 0;
 }
 
+static_assert(sizeof(ClosestPlan) <= 32, "a listed ray's plan takes 32 bytes");
+
+// The objects of an extension ray of a scene with one mesh (closest_plan): a ray that needs no tree walk is
+// finished here (its hit record written), the others are compacted into the walk list for
+// k_extend_refill, so that its lanes only ever hold rays that walk.  Every lane of the warp calls it;
+// valid: the lane has a ray, in queue slot i.
+template <int N>
+__device__ __forceinline__ void plan_ray(const DevScene<N>& S, const Ray<N>& r, bool valid, long long i, const HitView<N>& H,
+                                         int* __restrict__ list, ClosestPlan* __restrict__ plans,
+                                         unsigned long long* counters)
+{
+        bool walk = false;
+        ClosestPlan plan;
+        if (valid)
+        {
+                closest_plan<N>(S, r, &plan);
+                walk = plan.walk;
+                if (!walk)
+                {
+                        if (plan.pre_obj >= 0)
+                        {
+                                H.t[i] = plan.pre_t;
+                                H.obj[i] = plan.pre_obj;
+                                H.facet[i] = -1;
+                        }
+                        else
+                        {
+                                H.obj[i] = -1;
+                        }
+                }
+        }
+        const long long q = compact_slot(walk, counters + C_WALK_EXT);
+        if (q >= 0)
+        {
+                list[q] = (int)i;
+                plans[q] = plan;
+        }
+}
+
+// Scenes with one mesh: the fresh rays are planned here too, in registers.
 template <int N>
 __global__ void __launch_bounds__(BLOCK) k_raygen(__grid_constant__ const DevScene<N> S, const PassDev P, PathView<N> A,
-                                                  const unsigned long long* __restrict__ ctl)
+                                                  HitView<N> H, int* __restrict__ list, ClosestPlan* __restrict__ plans,
+                                                  unsigned long long* counters)
 {
-        // this iteration's fresh paths (k_iter_begin): queue slots base.., pass paths first..
-        const long long fresh = (long long)ctl[C_Q_FRESH];
-        const long long base = (long long)ctl[C_Q_BASE];
-        const long long first = (long long)ctl[C_Q_NEXT] - fresh;
-        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < fresh; i += (long long)gridDim.x * blockDim.x)
+        // this iteration's fresh paths (iteration_begin): queue slots base.., pass paths first..
+        const long long fresh = (long long)counters[C_Q_FRESH];
+        const long long base = (long long)counters[C_Q_BASE];
+        const long long first = (long long)counters[C_Q_NEXT] - fresh;
+        const bool one_mesh = S.nmesh == 1;
+        const int lane = threadIdx.x & 31;
+        const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+        long long rays = 0;
+        for (long long w0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; w0 < fresh;
+             w0 += warps * 32)
         {
-                raygen_one<N>(S, P, A, P.path_begin + first + i, base + i);
+                const long long i = w0 + lane;
+                const bool valid = i < fresh;
+                Ray<N> r;
+                if (valid)
+                {
+                        raygen_one<N>(S, P, A, P.path_begin + first + i, base + i, r);
+                        ++rays;
+                }
+                if (one_mesh)
+                {
+                        plan_ray<N>(S, r, valid, base + i, H, list, plans, counters);
+                }
+        }
+        if (one_mesh)
+        {
+                warp_add(counters + C_RAYS, rays);
         }
 }
 
@@ -413,6 +470,7 @@ __global__ void __launch_bounds__(BLOCK, shade_min_blocks<N>()) k_shade(__grid_c
                                                  unsigned long long* counters, int parity)
 {
         const long long count = (long long)counters[C_Q_ACTIVE];
+        const long long continuing = (long long)counters[C_Q_BASE];  // the paths from there on are fresh
         __shared__ CompactShared s_compact;
         int turn = 0;
         const bool one_mesh = S.nmesh == 1;
@@ -435,11 +493,16 @@ __global__ void __launch_bounds__(BLOCK, shade_min_blocks<N>()) k_shade(__grid_c
                 {
                         pixel = A.pix[i];
                         sample = A.smp[i];
-                        level = A.level[i];
-                        beta[0] = A.at(2 * N + 0, i);
-                        beta[1] = A.at(2 * N + 1, i);
-                        beta[2] = A.at(2 * N + 2, i);
-                        float color_level = A.at(2 * N + 3, i);
+                        float color_level = 1.0f;
+                        beta[0] = beta[1] = beta[2] = 1.0f;
+                        if (i < continuing)
+                        {
+                                level = A.level[i];
+                                beta[0] = A.at(2 * N + 0, i);
+                                beta[1] = A.at(2 * N + 1, i);
+                                beta[2] = A.at(2 * N + 2, i);
+                                color_level = A.at(2 * N + 3, i);
+                        }
                         Ray<N> ray;
 #pragma unroll
                         for (int k = 0; k < N; ++k)
@@ -843,17 +906,13 @@ __device__ __forceinline__ long long lane_refill(bool idle, unsigned long long* 
         return j < count ? j : -1;
 }
 
-static_assert(sizeof(ClosestPlan) <= 32, "a listed ray's plan takes 32 bytes");
-
-// Extension rays of a scene with one mesh, first pass: every ray's objects (closest_plan); the rays
-// that need no tree walk are finished here (their hit record written), the others are compacted into
-// the walk list for k_extend_refill, so that its lanes only ever hold rays that walk.
+// The continuing extension rays of a scene with one mesh (the queue's slots below C_Q_BASE), first pass.
 template <int N>
 __global__ void __launch_bounds__(BLOCK) k_plan_extend(__grid_constant__ const DevScene<N> S, PathView<N> A, HitView<N> H,
                                                        int* __restrict__ list, ClosestPlan* __restrict__ plans,
                                                        unsigned long long* counters)
 {
-        const long long count = (long long)counters[C_Q_ACTIVE];
+        const long long count = (long long)counters[C_Q_BASE];
         const int lane = threadIdx.x & 31;
         const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
         long long rays = 0;
@@ -861,40 +920,19 @@ __global__ void __launch_bounds__(BLOCK) k_plan_extend(__grid_constant__ const D
              w0 += warps * 32)
         {
                 const long long i = w0 + lane;
-                bool walk = false;
-                ClosestPlan plan;
-                if (i < count)
+                const bool valid = i < count;
+                Ray<N> r;
+                if (valid)
                 {
                         ++rays;
-                        Ray<N> r;
 #pragma unroll
                         for (int k = 0; k < N; ++k)
                         {
                                 r.org[k] = A.at(k, i);
                                 r.dir[k] = A.at(N + k, i);
                         }
-                        closest_plan<N>(S, r, &plan);
-                        walk = plan.walk;
-                        if (!walk)
-                        {
-                                if (plan.pre_obj >= 0)
-                                {
-                                        H.t[i] = plan.pre_t;
-                                        H.obj[i] = plan.pre_obj;
-                                        H.facet[i] = -1;
-                                }
-                                else
-                                {
-                                        H.obj[i] = -1;
-                                }
-                        }
                 }
-                const long long q = compact_slot(walk, counters + C_WALK_EXT);
-                if (q >= 0)
-                {
-                        list[q] = (int)i;
-                        plans[q] = plan;
-                }
+                plan_ray<N>(S, r, valid, i, H, list, plans, counters);
         }
         warp_add(counters + C_RAYS, rays);
 }
@@ -1370,7 +1408,7 @@ void Wavefront<N>::enqueue_iteration(const DevScene<N>& S, const PassDev& P, dou
         {
                 cudaEventRecord(ev[0], st);
         }
-        k_raygen<N><<<raygen_grid, BLOCK, 0, st>>>(S, P, A, counters);
+        k_raygen<N><<<raygen_grid, BLOCK, 0, st>>>(S, P, A, H, walk_ext, (ClosestPlan*)plan_ext, counters);
         if (ev)
         {
                 cudaEventRecord(ev[1], st);

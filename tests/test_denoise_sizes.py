@@ -1,0 +1,55 @@
+"""The denoiser's kernels at the sizes where they could go wrong: pixel counts around the inference
+kernel's 128-pixel tiles and past one tile per resident block, and row counts around the weight
+gradients' 256 rows per block, against the numpy oracle with the same BF16 rounding points."""
+
+import numpy as np
+import pytest
+
+from oracle import denoise_oracle as dor
+from test_denoise import SPP, _random_inputs, _random_params
+
+pytestmark = pytest.mark.gpu
+
+
+def _setup(n, screen, seed):
+    import torch
+
+    from math_b200.denoise import Denoiser
+
+    rng = np.random.default_rng(seed)
+    host = _random_inputs(n, screen, rng)
+    params = _random_params(n, rng).astype(np.float32)
+    den = Denoiser(n, seed=0)
+    den.set_params(params)
+    dev = [torch.from_numpy(a).cuda() for a in host]
+    den.set_input(screen, *dev[:4], SPP)
+    return den, params, host, dev
+
+
+@pytest.mark.parametrize("n,screen", [(3, (1, 1)), (3, (127, 1)), (3, (128, 1)), (3, (43, 3)), (4, (5, 17, 3)),
+                                      (5, (4, 5, 2, 7)), (6, (2, 3, 5, 2, 9)), (3, (251, 229))])
+def test_inference_matches_the_oracle_around_tile_edges(require_gpu, n, screen):
+    """(251, 229): 57,479 pixels, more tiles than resident blocks, the last one ragged."""
+    den, params, (mean, var, normal, depth, _), _ = _setup(n, screen, 5)
+    out = den.apply().cpu().numpy()
+    want = dor.forward(params, n, screen, mean, var, normal, depth, spp=SPP, bf16_points=True)["out"]
+    # FP32 sums in another order move a BF16 rounding of a hidden value by one unit (2^-8) here and there:
+    # the output, a weighted mean of pixels, by far less (the tests of the same network use 2e-3)
+    assert np.linalg.norm(out - want) <= 2e-3 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("screen", [(255, 1), (256, 1), (257, 1), (97, 11)])
+def test_gradients_match_the_oracle_around_the_split_of_the_rows(require_gpu, screen):
+    n = 3
+    den, params, (mean, var, normal, depth, target), dev = _setup(n, screen, 6)
+    loss, grad = den.gradient(dev[4])
+    want_loss, want = dor.loss_and_grad(params, n, screen, mean, var, normal, depth, target, spp=SPP, bf16_points=True)
+    assert abs(loss - want_loss) <= 2e-3 * want_loss
+    got, ref = dor.split(grad, n), dor.split(want, n)
+    for name in got:
+        # each block within the 2e-2 of the network's other gradient tests (BF16 products)
+        assert np.linalg.norm(got[name] - ref[name]) <= 2e-2 * np.linalg.norm(ref[name]), name
+    # and inference after a training pass of the same input gives the forward pass's image
+    out = den.apply().cpu().numpy()
+    fwd = dor.forward(params, n, screen, mean, var, normal, depth, spp=SPP, bf16_points=True)["out"]
+    assert np.linalg.norm(out - fwd) <= 2e-3 * np.linalg.norm(fwd)
