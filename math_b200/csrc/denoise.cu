@@ -1408,6 +1408,10 @@ struct nt_denoiser
         Stencil st{};
         cudaStream_t own = nullptr;
         cudaStream_t st_use = nullptr;
+        // the weight gradients that the backward chain does not wait for, and the events that tie their
+        // stream to st_use
+        cudaStream_t side = nullptr;
+        cudaEvent_t fork = nullptr, join = nullptr;
         long long adam_t = 0;
         // parameters and optimiser state (flat FP32), packed weights
         Buf w, g, m, v;
@@ -1578,35 +1582,40 @@ double backward(nt_denoiser* d, const float* target)
                 std::swap(gout, gin);
         }
         ck(cudaGetLastError(), "filter backward");
-        // backward data products
-        ck(gemm(LoadRows{d->dZ, d->Op}, LoadCols{d->W3.as<__nv_bfloat16>(), HID},
-                EpiMaskBF16{d->H2, d->dH2, HID}, P32, HID, d->Op, 0, err, s),
-           "gemm dH2");
-        ck(gemm(LoadRows{d->dH2, HID}, LoadCols{d->W2.as<__nv_bfloat16>(), HID},
-                EpiMaskBF16{d->H1, d->dH1, HID}, P32, HID, HID, 0, err, s),
-           "gemm dH1");
-        // weight gradients: reductions over pixels, split across CTAs, about four per SM (the products
-        // are skinny and HBM-bound, so their copies need the CTAs in flight)
+        // Backward data products and weight gradients.  The weight gradients are reductions over pixels, split
+        // across CTAs, about four per SM (the products are skinny and HBM-bound, so their copies need the CTAs
+        // in flight), at least 256 rows each: every CTA adds its whole matrix to the sum with atomics.  Over
+        // few pixels each leaves most SMs idle, so those that the chain dZ -> dH2 -> dH1 does not wait for run
+        // beside it on the side stream.
         ck(cudaMemsetAsync(d->gblock.p, 0, d->gbytes(), s), "memset");
         int dev = 0, sms = 148;
         ck(cudaGetDevice(&dev), "device");
         ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
-        // at least 256 rows each: every CTA adds its whole matrix to the sum with atomics
         const long long ctas = 4LL * std::max(1, sms);
         const int kpc = (int)std::max<long long>(4 * GK, ((long long)P32 + ctas - 1) / ctas);
-        ck(gemm(LoadCols{d->dZ, d->Op}, LoadCols{d->H2, HID},
-                EpiAtomicF32{d->gW3, HID, HID}, d->Op, HID, P32, kpc, err, s),
+        auto fork = [&]() {
+                ck(cudaEventRecord(d->fork, s), "event");
+                ck(cudaStreamWaitEvent(d->side, d->fork, 0), "event");
+        };
+        fork();
+        ck(gemm(LoadCols{d->dZ, d->Op}, LoadCols{d->H2, HID}, EpiAtomicF32{d->gW3, HID, HID}, d->Op, HID, P32, kpc, err, d->side),
            "gemm dW3");
-        ck(gemm(LoadCols{d->dH2, HID}, LoadCols{d->H1, HID},
-                EpiAtomicF32{d->gW2, HID, HID}, HID, HID, P32, kpc, err, s),
+        ck(gemm(LoadRows{d->dZ, d->Op}, LoadCols{d->W3.as<__nv_bfloat16>(), HID}, EpiMaskBF16{d->H2, d->dH2, HID}, P32, HID, d->Op,
+                0, err, s),
+           "gemm dH2");
+        fork();
+        ck(gemm(LoadCols{d->dH2, HID}, LoadCols{d->H1, HID}, EpiAtomicF32{d->gW2, HID, HID}, HID, HID, P32, kpc, err, d->side),
            "gemm dW2");
-        ck(gemm(LoadCols{d->dH1, HID}, LoadCols{d->X, d->Fp},
-                EpiAtomicF32{d->gW1, d->Fp, d->Fp}, HID, d->Fp, P32, kpc, err, s),
+        ck(gemm(LoadRows{d->dH2, HID}, LoadCols{d->W2.as<__nv_bfloat16>(), HID}, EpiMaskBF16{d->H1, d->dH1, HID}, P32, HID, HID, 0,
+                err, s),
+           "gemm dH1");
+        fork();
+        const ColSums cs{{d->dZ, d->dH2, d->dH1}, {d->gb3, d->gb2, d->gb1}, {d->Op, HID, HID}};
+        k_colsum<<<dim3((unsigned)std::min<long long>((P + 127) / 128, 256), 3), TB, 0, d->side>>>(P, cs);
+        ck(cudaEventRecord(d->join, d->side), "event");
+        ck(gemm(LoadCols{d->dH1, HID}, LoadCols{d->X, d->Fp}, EpiAtomicF32{d->gW1, d->Fp, d->Fp}, HID, d->Fp, P32, kpc, err, s),
            "gemm dW1");
-        const ColSums cs{{d->dZ, d->dH2, d->dH1},
-                         {d->gb3, d->gb2, d->gb1},
-                         {d->Op, HID, HID}};
-        k_colsum<<<dim3((unsigned)std::min<long long>((P + 127) / 128, 256), 3), TB, 0, s>>>(P, cs);
+        ck(cudaStreamWaitEvent(s, d->join, 0), "event");
         k_unpack<<<64, TB, 0, s>>>(d->F, d->Fp, d->O, d->gW1, d->gb1, d->gW2,
                                    d->gb2, d->gW3, d->gb3, d->g.as<float>());
         ck(cudaGetLastError(), "gradients");
@@ -1659,6 +1668,9 @@ int nt_denoiser_create(int n, uint64_t seed, nt_denoiser** out)
                 d->nparams = (long long)HID * d->F + HID + HID * HID + HID + (long long)d->O * HID + d->O;
                 ck(cudaStreamCreateWithFlags(&d->own, cudaStreamNonBlocking), "cudaStreamCreate");
                 d->st_use = d->own;
+                ck(cudaStreamCreateWithFlags(&d->side, cudaStreamNonBlocking), "cudaStreamCreate");
+                ck(cudaEventCreateWithFlags(&d->fork, cudaEventDisableTiming), "cudaEventCreate");
+                ck(cudaEventCreateWithFlags(&d->join, cudaEventDisableTiming), "cudaEventCreate");
                 const size_t pb = sizeof(float) * (size_t)d->nparams;
                 d->w.ensure(pb);
                 d->g.ensure(pb);
@@ -1717,10 +1729,20 @@ int nt_denoiser_destroy(nt_denoiser* d)
         {
                 return NT_OK;
         }
-        if (d->own)
+        for (cudaStream_t t : {d->own, d->side})
         {
-                cudaStreamSynchronize(d->own);
-                cudaStreamDestroy(d->own);
+                if (t)
+                {
+                        cudaStreamSynchronize(t);
+                        cudaStreamDestroy(t);
+                }
+        }
+        for (cudaEvent_t e : {d->fork, d->join})
+        {
+                if (e)
+                {
+                        cudaEventDestroy(e);
+                }
         }
         delete d;
         return NT_OK;
