@@ -1699,7 +1699,7 @@ __device__ __forceinline__ int pool_closest(const MeshDev<N>& M, const WarpPool&
                                 continue;
                         }
                         __syncwarp();
-                        // the owner's sequential choice over its hits of this round, in list order
+                        // the owner's sequential choice over its hits among these tests, in list order
                         const int q0 = min(max(P.excl - base, 0), 32);
                         const int q1 = min(max(P.excl + P.cnt - base, 0), 32);
                         unsigned mine = hits & (unsigned)((1ull << q1) - (1ull << q0));

@@ -1538,10 +1538,14 @@ void Wavefront<N>::enqueue_iterations(const DevScene<N>& S, const PassDev& P, do
                                       long long total_paths, int count, cudaStream_t st, KernelTimes* times,
                                       const SideStream* side) const
 {
+        const bool smooth = S.smooth_normal != 0;
         if (side)
         {
                 cudaEventRecord(side->join, st);
-                cudaEventRecord(side->join_smooth, st);
+                if (smooth)
+                {
+                        cudaEventRecord(side->join_smooth, st);
+                }
         }
         for (int k = 0; k < count; ++k)
         {
@@ -1550,7 +1554,10 @@ void Wavefront<N>::enqueue_iterations(const DevScene<N>& S, const PassDev& P, do
         if (side)
         {
                 cudaStreamWaitEvent(st, side->join, 0);
-                cudaStreamWaitEvent(st, side->join_smooth, 0);
+                if (smooth)
+                {
+                        cudaStreamWaitEvent(st, side->join_smooth, 0);
+                }
         }
 }
 

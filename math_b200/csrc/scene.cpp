@@ -1084,10 +1084,7 @@ void build_scene(nt_scene* s, unsigned threads, bool host_only, bool tree_on_gpu
         }
         if (!host_only && !s->join2)
         {
-                for (cudaStream_t* t : {&s->side.stream, &s->side.smooth, &s->stream2, &s->side2.stream, &s->side2.smooth})
-                {
-                        check_cuda(cudaStreamCreateWithFlags(t, cudaStreamNonBlocking), "cudaStreamCreate");
-                }
+                check_cuda(cudaStreamCreateWithFlags(&s->side.stream, cudaStreamNonBlocking), "cudaStreamCreate");
                 for (cudaEvent_t* e : {&s->side.fork, &s->side.join, &s->side.join_smooth, &s->side2.fork, &s->side2.join,
                                        &s->side2.join_smooth, &s->fork2, &s->join2})
                 {
@@ -1611,10 +1608,40 @@ std::unique_ptr<PassJob> prepare_pass(nt_scene* s, const nt_render_opts& o, cons
         // that for two halves
         const long long per_path =
                 (long long)(Wavefront<N>::bytes_for(1, lights, smooth) - Wavefront<N>::bytes_for(0, lights, smooth));
-        const long long automatic = std::min<long long>(1ll << 22, (1ll << 30) / per_path) * (job->halves ? 2 : 1);
-        long long Q = o.pool_paths > 0 ? o.pool_paths : automatic;
+        const long long whole = std::min<long long>(1ll << 22, (1ll << 30) / per_path);
+        long long Q = o.pool_paths > 0 ? o.pool_paths : (job->halves ? 2 * whole : whole);
+        if (o.pool_paths <= 0 && job->halves && Q > s->pool_paths)
+        {
+                // the larger pool only where it fits beside what the device holds
+                size_t free_b = 0, total_b = 0;
+                check_cuda(cudaMemGetInfo(&free_b, &total_b), "memory info");
+                if (Wavefront<N>::bytes_for(Q, lights, smooth) + (64u << 20) > free_b + s->pool.bytes)
+                {
+                        Q = whole;
+                }
+        }
         Q = std::max<long long>(256, std::min(Q, total));
         job->halves = job->halves && Q >= HALVES_PATHS;
+        // the streams that not every scene needs, made by the first pass that does
+        auto need = [](cudaStream_t* t) {
+                if (!*t)
+                {
+                        check_cuda(cudaStreamCreateWithFlags(t, cudaStreamNonBlocking), "cudaStreamCreate");
+                }
+        };
+        if (smooth)
+        {
+                need(&s->side.smooth);
+        }
+        if (job->halves)
+        {
+                need(&s->stream2);
+                need(&s->side2.stream);
+                if (smooth)
+                {
+                        need(&s->side2.smooth);
+                }
+        }
         if (Q > s->pool_paths || lights > s->pool_lights || (smooth && !s->pool_smooth))
         {
                 // (the fixed part twice: two halves are two pools)
