@@ -213,7 +213,7 @@ void build_tree_gpu(const std::vector<SimplexShape<N, float>>& shapes, const Vec
         const long long nf = (long long)shapes.size();
         constexpr int C = 1 << N;
         Dev d_shapes;
-        Dev d_kids, d_bits, d_counts, d_off, d_child;  // a level's work memory, kept for the next one
+        Dev d_work;  // a level's work memory, one allocation, kept for the next one
         TB_CHECK(d_shapes.alloc(sizeof(SimplexShape<N, float>) * (size_t)nf), "cudaMalloc");
         TB_CHECK(cudaMemcpyAsync(d_shapes.p, shapes.data(), sizeof(SimplexShape<N, float>) * (size_t)nf,
                                  cudaMemcpyHostToDevice, st),
@@ -302,26 +302,33 @@ void build_tree_gpu(const std::vector<SimplexShape<N, float>>& shapes, const Vec
                                 tests += (unsigned long long)parent.cnt;
                         }
                 }
-                TB_CHECK(d_kids.alloc(sizeof(ChildDesc<N>) * (size_t)nkids), "cudaMalloc");
-                TB_CHECK(d_bits.alloc(sizeof(unsigned) * (size_t)words), "cudaMalloc");
-                TB_CHECK(d_counts.alloc(sizeof(unsigned) * (size_t)nkids), "cudaMalloc");
-                TB_CHECK(cudaMemcpyAsync(d_kids.p, kids.data(), sizeof(ChildDesc<N>) * (size_t)nkids, cudaMemcpyHostToDevice,
+                auto padded = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+                const size_t kb = padded(sizeof(ChildDesc<N>) * (size_t)nkids), ob = padded(sizeof(long long) * (size_t)nkids);
+                const size_t cb = padded(sizeof(unsigned) * (size_t)nkids), wb = padded(sizeof(unsigned) * (size_t)words);
+                // (room for the next level at once: an allocation takes a tenth of a millisecond and more)
+                if (kb + ob + cb + 2 * wb > d_work.bytes)
+                {
+                        TB_CHECK(d_work.alloc(std::max(kb + ob + cb + 2 * wb, 2 * d_work.bytes)), "cudaMalloc");
+                }
+                char* const work = static_cast<char*>(d_work.p);
+                ChildDesc<N>* const d_kids = reinterpret_cast<ChildDesc<N>*>(work);
+                long long* const d_off = reinterpret_cast<long long*>(work + kb);
+                unsigned* const d_counts = reinterpret_cast<unsigned*>(work + kb + ob);
+                unsigned* const d_bits = reinterpret_cast<unsigned*>(work + kb + ob + cb);
+                int* const d_child = reinterpret_cast<int*>(work + kb + ob + cb + wb);
+                TB_CHECK(cudaMemcpyAsync(d_kids, kids.data(), sizeof(ChildDesc<N>) * (size_t)nkids, cudaMemcpyHostToDevice,
                                          st),
                          "upload");
-                TB_CHECK(d_child.alloc(sizeof(int) * (size_t)words), "cudaMalloc");
-                TB_CHECK(cudaMemsetAsync(d_counts.p, 0, sizeof(unsigned) * (size_t)nkids, st), "memset");
+                TB_CHECK(cudaMemsetAsync(d_counts, 0, sizeof(unsigned) * (size_t)nkids, st), "memset");
                 const unsigned cgrid = (unsigned)std::min<long long>((nkids + TB / 32 - 1) / (TB / 32), 148LL * 64);
-                k_word_child<N><<<cgrid, TB, 0, st>>>(static_cast<const ChildDesc<N>*>(d_kids.p), nkids,
-                                                      static_cast<int*>(d_child.p));
+                k_word_child<N><<<cgrid, TB, 0, st>>>(d_kids, nkids, d_child);
                 const unsigned grid = (unsigned)std::min<long long>((words + TB / 32 - 1) / (TB / 32), 148LL * 16);
                 k_overlap<N><<<grid, TB, 0, st>>>(static_cast<const SimplexShape<N, float>*>(d_shapes.p),
-                                                  static_cast<const int*>(lists[level]->p),
-                                                  static_cast<const ChildDesc<N>*>(d_kids.p),
-                                                  static_cast<const int*>(d_child.p), words, half,
-                                                  static_cast<unsigned*>(d_bits.p), static_cast<unsigned*>(d_counts.p));
+                                                  static_cast<const int*>(lists[level]->p), d_kids, d_child, words, half,
+                                                  d_bits, d_counts);
                 TB_CHECK(cudaGetLastError(), "overlap kernel");
                 std::vector<unsigned> counts((size_t)nkids);
-                TB_CHECK(cudaMemcpyAsync(counts.data(), d_counts.p, sizeof(unsigned) * (size_t)nkids, cudaMemcpyDeviceToHost,
+                TB_CHECK(cudaMemcpyAsync(counts.data(), d_counts, sizeof(unsigned) * (size_t)nkids, cudaMemcpyDeviceToHost,
                                          st),
                          "copy");
                 TB_CHECK(cudaStreamSynchronize(st), "overlap");
@@ -332,17 +339,13 @@ void build_tree_gpu(const std::vector<SimplexShape<N, float>>& shapes, const Vec
                         off[c] = total;
                         total += counts[c];
                 }
-                TB_CHECK(d_off.alloc(sizeof(long long) * (size_t)nkids), "cudaMalloc");
-                TB_CHECK(cudaMemcpyAsync(d_off.p, off.data(), sizeof(long long) * (size_t)nkids, cudaMemcpyHostToDevice, st),
-                         "upload");
+                TB_CHECK(cudaMemcpyAsync(d_off, off.data(), sizeof(long long) * (size_t)nkids, cudaMemcpyHostToDevice, st), "upload");
                 lists.push_back(std::make_unique<Dev>());
                 TB_CHECK(lists.back()->alloc(sizeof(int) * (size_t)total), "cudaMalloc");
                 list_sizes.push_back(total);
                 const unsigned wgrid = (unsigned)std::min<long long>((nkids + TB / 32 - 1) / (TB / 32), 148LL * 64);
-                k_write<N><<<wgrid, TB, 0, st>>>(static_cast<const int*>(lists[level]->p),
-                                                 static_cast<const ChildDesc<N>*>(d_kids.p), nkids,
-                                                 static_cast<const unsigned*>(d_bits.p),
-                                                 static_cast<const long long*>(d_off.p), static_cast<int*>(lists.back()->p));
+                k_write<N><<<wgrid, TB, 0, st>>>(static_cast<const int*>(lists[level]->p), d_kids, nkids, d_bits, d_off,
+                                                 static_cast<int*>(lists.back()->p));
                 TB_CHECK(cudaGetLastError(), "write kernel");
                 TB_CHECK(cudaStreamSynchronize(st), "write");
                 std::vector<BoxRef> next((size_t)nkids);
